@@ -10,9 +10,9 @@
 //      into per-task global bins), one warp evaluates SAH over the 3 x 31
 //      planes, a chunked stable partition (block scans) reorders the refs;
 //   3. small tasks (<= kSmall): one block builds the whole subtree in shared
-//      memory, always descending into the smaller child so its stack stays
-//      <= log2(kSmall) deep; node ids come from a per-task reserved range, so
-//      the tree is deterministic;
+//      memory, a warp per node, nodes of at most 32 primitives one primitive
+//      per lane; a split's place among the refs names its children's node
+//      slots, so the tree is deterministic;
 //   4. collapse: a bottom-up pass fills the SAH cost table of the optimal
 //      collapse (k_dp_up); then breadth first, every wide node takes the 8
 //      children that table chose; children with at most 1 (large scenes) or 3
@@ -49,7 +49,6 @@ constexpr int kLeafLarge = 1;
 constexpr int kLargeSceneTris = 1 << 16;   // scenes above this use kLeafLarge
 constexpr int kThreads = 256;
 constexpr int kBinInts = 13;   // count, box lo/hi, centroid lo/hi (ordered ints)
-constexpr int kStack = 32;
 
 enum BuildError : int {
     kErrNone = 0,
@@ -408,206 +407,401 @@ __global__ void k_write_nodes(const int *ids, const BinNode *vals, const int *fi
 
 // ---------------------------------------------------------------------------
 // 3. small tasks: one block builds a whole subtree
+//
+// The block holds its task's primitive boxes in shared memory and permutes
+// 16-bit local indices.  Nodes of more than 32 primitives go level by level,
+// a warp (or, while a level has fewer nodes than the block has warps, a group
+// of warps) binning each; nodes of at most 32 are finished by one warp with a
+// primitive per lane (tiny_build).  A split at position m of the task (its
+// right child begins there) owns the node slots slot_base + 2 (m - 1) + {0, 1}:
+// every split of a task has its own m, so no counter orders the warps and the
+// tree is the same on every run.
+//
+// What bounds it: the binary tree down to one triangle has as many inner
+// nodes as triangles, half of them with two or three primitives.  One block
+// of 256 threads per node (its bins cleared, filled and scanned, eight
+// barriers, for two primitives) took 126.5 ms of the 142 ms build of 5.2M
+// triangles; this takes 3.55 ms (82k triangles: 10.2 -> 0.23 ms), the same
+// tree.  Shared-memory atomics bound the levels above 32 primitives, shuffles
+// and min / max the rest; boxes in shared memory (108 KB) allow two blocks of
+// 12 warps per SM, whose levels overlap.
 // ---------------------------------------------------------------------------
-struct SmallEntry {
-    int node, b, c, pad;
+constexpr int kSbWarps = 12, kSbThreads = 32 * kSbWarps;  // two blocks per SM (shared memory)
+constexpr int kTiny = 32;       // nodes up to this size: one primitive per lane
+constexpr int kSbBinInts = 7;   // count, box lo / hi (ordered ints)
+constexpr int kSbBins = 3 * kBins * kSbBinInts;
+constexpr int kSbNodes = kSmall / (kTiny + 1) + 1;  // nodes above kTiny primitives on one level
+
+struct SbNode {
+    int node, b, c;
     float clo[3], chi[3];
 };
 
-__global__ void __launch_bounds__(kThreads) k_small_build(const Task *tasks, const int *slot_base,
-                                                          const int *slot_end, int ntasks,
-                                                          const float4 *__restrict__ plo,
-                                                          const float4 *__restrict__ phi, int *ref,
-                                                          BinNode *nodes, int *bfirst, int *bcount,
-                                                          int cap, int max_leaf, int *err) {
-    __shared__ int sref[kSmall];
-    __shared__ int stmp[kSmall];
-    __shared__ int bins[3 * kBins * kBinInts];
-    __shared__ SmallEntry stack[kStack];
-    __shared__ int sp;
-    __shared__ int ws[32];
-    __shared__ WarpSplit best;
-    __shared__ SmallEntry cur;
-    __shared__ int next_slot;
-    __shared__ float red[kThreads / 32][12];
+struct SbShared {
+    float box[6][kSmall];          // lo xyz, hi xyz by local index
+    int prim[kSmall];              // primitive of a local index
+    unsigned short idx[kSmall], tmp[kSmall];
+    int bins[kSbWarps][kSbBins];
+    SbNode list[2][kSbNodes];      // this level's and the next level's nodes
+    int2 tiny[kSmall / 2];         // (node, b | c << 16)
+    unsigned char perm[kSbWarps][32];
+    int n_list[2], n_tiny;
+};
+static_assert(2 * (sizeof(SbShared) + 1024) <= 227 * 1024, "two blocks per SM");
 
-    const int t = blockIdx.x;
-    if (t >= ntasks) return;
-    const Task tk = tasks[t];
-    if (tk.count > kSmall || tk.count < 1) {
-        if (threadIdx.x == 0) raise_err(err, kErrSmallTooBig);
+// What the build writes of a node when it is made: its box and its range of
+// refs; a leaf's mark, or links that its own split fills in.
+__device__ __forceinline__ void put_node(BinNode *nodes, int *bfirst, int *bcount, int id, float3 lo, float3 hi,
+                                         int first, int count, bool leaf) {
+    nodes[id].lo = make_float4(lo.x, lo.y, lo.z, leaf ? __int_as_float(first) : 0.0f);
+    nodes[id].hi = make_float4(hi.x, hi.y, hi.z, leaf ? __int_as_float(-count) : 0.0f);
+    bfirst[id] = first;
+    bcount[id] = count;
+}
+
+__device__ __forceinline__ float3 warp_min3(float3 v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        v = fmin3(v, f3(__shfl_xor_sync(~0u, v.x, o), __shfl_xor_sync(~0u, v.y, o), __shfl_xor_sync(~0u, v.z, o)));
+    return v;
+}
+__device__ __forceinline__ float3 warp_max3(float3 v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        v = fmax3(v, f3(__shfl_xor_sync(~0u, v.x, o), __shfl_xor_sync(~0u, v.y, o), __shfl_xor_sync(~0u, v.z, o)));
+    return v;
+}
+__device__ __forceinline__ float3 shfl3(float3 v, int src) {
+    return f3(__shfl_sync(~0u, v.x, src), __shfl_sync(~0u, v.y, src), __shfl_sync(~0u, v.z, src));
+}
+
+// warp_best_split over a warp's bins of kSbBinInts ints (no centroid boxes);
+// also the number of primitives left of the plane.
+__device__ WarpSplit sb_best_split(const int *bins, int *n_left) {
+    const int lane = threadIdx.x & 31;
+    WarpSplit best{-1, -1, INFINITY};
+    int nl = 0;
+    for (int a = 0; a < 3; ++a) {
+        const int *B = bins + (a * kBins + lane) * kSbBinInts;
+        int pc = B[0], sc = pc;
+        float3 plo = f3(o2f(B[1]), o2f(B[2]), o2f(B[3])), phi = f3(o2f(B[4]), o2f(B[5]), o2f(B[6]));
+        float3 slo = plo, shi = phi;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(~0u, pc, o), d = __shfl_down_sync(~0u, sc, o);
+            const float3 ulo = shfl_up3(plo, o), uhi = shfl_up3(phi, o);
+            const float3 dlo = shfl_down3(slo, o), dhi = shfl_down3(shi, o);
+            if (lane >= o) { pc += u; plo = fmin3(plo, ulo); phi = fmax3(phi, uhi); }
+            if (lane + o < 32) { sc += d; slo = fmin3(slo, dlo); shi = fmax3(shi, dhi); }
+        }
+        const int rc = __shfl_down_sync(~0u, sc, 1);
+        const float3 rlo = shfl_down3(slo, 1), rhi = shfl_down3(shi, 1);
+        float c = INFINITY;
+        if (lane < 31 && pc > 0 && rc > 0)
+            c = surface_area(plo, phi) * (float)pc + surface_area(rlo, rhi) * (float)rc;
+        int l = lane;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float c2 = __shfl_xor_sync(~0u, c, o);
+            const int l2 = __shfl_xor_sync(~0u, l, o);
+            if (c2 < c || (c2 == c && l2 < l)) { c = c2; l = l2; }
+        }
+        const int lc = __shfl_sync(~0u, pc, l);
+        if (c < best.cost) { best.cost = c; best.axis = a; best.bin = l; nl = lc; }
+    }
+    *n_left = nl;
+    return best;
+}
+
+// Finishes the subtree of at most 32 primitives at refs [b, b + c) of the
+// task: lane i holds primitive i, the nodes of one level are segments of
+// lanes, and all of them are split at once.  A segment's candidate planes are
+// its primitives' own bins (an empty bin's plane makes the same partition as
+// the occupied bin before it, at a larger index), so lane i sums the boxes
+// left and right of its bin on each axis by walking its segment; the choice
+// (least cost, then lowest axis, then lowest bin) is that of the 32-bin scan.
+__device__ void tiny_build(SbShared &sh, int root, int b, int c, int begin, int slot_base, int max_leaf,
+                           BinNode *nodes, int *bfirst, int *bcount) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    const bool mine = lane < c;
+    int local = mine ? sh.idx[b + lane] : 0;
+    float3 lo = f3(sh.box[0][local], sh.box[1][local], sh.box[2][local]);
+    float3 hi = f3(sh.box[3][local], sh.box[4][local], sh.box[5][local]);
+    int sb = mine ? 0 : lane, se = mine ? c : lane + 1;  // this lane's segment
+    int node = root;
+    while (true) {
+        const int s = se - sb;
+        const bool act = mine && s > max_leaf;
+        const int longest = __reduce_max_sync(~0u, act ? s : 0);
+        if (longest == 0) break;
+        const float3 cen = f3(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z));
+        float3 clo = cen, chi = cen;
+        for (int k = 0; k < longest; ++k) {
+            const float3 q = shfl3(cen, min(sb + k, se - 1));
+            clo = fmin3(clo, q);
+            chi = fmax3(chi, q);
+        }
+        unsigned bin[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+            bin[a] = (unsigned)bin_of(comp(cen, a), comp(clo, a), bin_scale(comp(clo, a), comp(chi, a)));
+        const unsigned packed = bin[0] | bin[1] << 8 | bin[2] << 16;
+        float3 llo[3], lhi[3], rlo[3], rhi[3];
+        int lc[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            llo[a] = rlo[a] = f3(INFINITY, INFINITY, INFINITY);
+            lhi[a] = rhi[a] = f3(-INFINITY, -INFINITY, -INFINITY);
+            lc[a] = 0;
+        }
+        for (int k = 0; k < longest; ++k) {
+            // past the segment's end the last primitive again: boxes do not change, counts skip it
+            const int src = min(sb + k, se - 1), in = sb + k < se ? 1 : 0;
+            const float3 ql = shfl3(lo, src), qh = shfl3(hi, src);
+            const unsigned qb = __shfl_sync(~0u, packed, src);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                if (((qb >> (8 * a)) & 0xffu) <= bin[a]) {
+                    llo[a] = fmin3(llo[a], ql);
+                    lhi[a] = fmax3(lhi[a], qh);
+                    lc[a] += in;
+                } else {
+                    rlo[a] = fmin3(rlo[a], ql);
+                    rhi[a] = fmax3(rhi[a], qh);
+                }
+            }
+        }
+        float cost = INFINITY;
+        int key = 0x7fffffff;  // axis, bin
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const int rc = s - lc[a];
+            if (rc > 0) {
+                const float ca = surface_area(llo[a], lhi[a]) * (float)lc[a] + surface_area(rlo[a], rhi[a]) * (float)rc;
+                if (ca < cost) { cost = ca; key = a * kBins + (int)bin[a]; }
+            }
+        }
+        float best = cost;
+        int bkey = key;
+        for (int k = 0; k < longest; ++k) {
+            const int src = min(sb + k, se - 1);
+            const float q = __shfl_sync(~0u, cost, src);
+            const int qk = __shfl_sync(~0u, key, src);
+            if (q < best || (q == best && qk < bkey)) { best = q; bkey = qk; }
+        }
+        // no plane (all centroids in one bin on every axis): by position
+        bool left = lane - sb < s / 2;
+        if (best < INFINITY) {
+            const int a = bkey / kBins;
+            left = (a == 0 ? bin[0] : a == 1 ? bin[1] : bin[2]) <= (unsigned)(bkey % kBins);
+        }
+        const unsigned lefts = __ballot_sync(~0u, act && left);
+        const unsigned seg = (unsigned)((1ull << se) - (1ull << sb));
+        const int nl = __popc(lefts & seg);
+        const int dst = !act ? lane
+                        : left ? sb + __popc(lefts & seg & below) : sb + nl + __popc(~lefts & seg & below);
+        sh.perm[warp][dst] = (unsigned char)lane;
+        __syncwarp();
+        const int src = sh.perm[warp][lane];
+        __syncwarp();
+        lo = shfl3(lo, src);
+        hi = shfl3(hi, src);
+        local = __shfl_sync(~0u, local, src);
+        // the children's segments, boxes and records
+        const int mid = sb + nl, id = slot_base + 2 * (b + mid - 1);
+        const bool right = lane >= mid;
+        if (act) {
+            if (lane == sb) {
+                nodes[node].lo.w = __int_as_float(id);
+                nodes[node].hi.w = __int_as_float(id + 1);
+            }
+            node = right ? id + 1 : id;
+            sb = right ? mid : sb;
+            se = right ? se : mid;
+        }
+        float3 nlo = lo, nhi = hi;
+        const int longest2 = __reduce_max_sync(~0u, act ? se - sb : 0);
+        for (int k = 0; k < longest2; ++k) {
+            const int q = min(sb + k, se - 1);
+            nlo = fmin3(nlo, shfl3(lo, q));
+            nhi = fmax3(nhi, shfl3(hi, q));
+        }
+        if (act && lane == sb)
+            put_node(nodes, bfirst, bcount, node, nlo, nhi, begin + b + sb, se - sb, se - sb <= max_leaf);
+    }
+    if (mine) sh.idx[b + lane] = (unsigned short)local;
+}
+
+// Splits node e by its bins, one warp: the stable partition of its indices,
+// the children's boxes and centroid bounds, their records, and their places
+// in the next level's list or the tiny list.
+__device__ void sb_split(SbShared &sh, const SbNode &e, const int *bins, int next, int begin, int slot_base,
+                         int max_leaf, BinNode *nodes, int *bfirst, int *bcount, int *err) {
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    int nl;
+    const WarpSplit w = sb_best_split(bins, &nl);
+    if (w.axis < 0) nl = e.c / 2;
+    const int ax = w.axis < 0 ? 0 : w.axis;
+    const float sc = bin_scale(e.clo[ax], e.chi[ax]);
+    const float3 inf = f3(INFINITY, INFINITY, INFINITY), ninf = f3(-INFINITY, -INFINITY, -INFINITY);
+    float3 lo[2] = {inf, inf}, hi[2] = {ninf, ninf}, clo[2] = {inf, inf}, chi[2] = {ninf, ninf};
+    int nls = 0, nrs = 0;
+    for (int base = 0; base < e.c; base += 32) {
+        const int i = base + lane;
+        const bool valid = i < e.c;
+        const int local = valid ? sh.idx[e.b + i] : 0;
+        const float3 l = f3(sh.box[0][local], sh.box[1][local], sh.box[2][local]);
+        const float3 h = f3(sh.box[3][local], sh.box[4][local], sh.box[5][local]);
+        const float3 c = f3(0.5f * (l.x + h.x), 0.5f * (l.y + h.y), 0.5f * (l.z + h.z));
+        const bool left = w.axis < 0 ? i < e.c / 2 : bin_of(comp(c, ax), e.clo[ax], sc) <= w.bin;
+        const unsigned lm = __ballot_sync(~0u, valid && left), rm = __ballot_sync(~0u, valid && !left);
+        if (valid) {
+            const int dst = left ? nls + __popc(lm & below) : nl + nrs + __popc(rm & below);
+            if (dst < e.c) sh.tmp[e.b + dst] = (unsigned short)local;
+            else raise_err(err, kErrBadChild);
+            if (left) {
+                lo[0] = fmin3(lo[0], l); hi[0] = fmax3(hi[0], h);
+                clo[0] = fmin3(clo[0], c); chi[0] = fmax3(chi[0], c);
+            } else {
+                lo[1] = fmin3(lo[1], l); hi[1] = fmax3(hi[1], h);
+                clo[1] = fmin3(clo[1], c); chi[1] = fmax3(chi[1], c);
+            }
+        }
+        nls += __popc(lm);
+        nrs += __popc(rm);
+    }
+    if (nls != nl) {  // the partition disagrees with the bins: no children
+        if (lane == 0) raise_err(err, kErrBadChild);
         return;
     }
-    const int m = tk.count;
-    for (int i = threadIdx.x; i < m; i += blockDim.x) sref[i] = ref[tk.begin + i];
+    __syncwarp();
+    for (int i = lane; i < e.c; i += 32) sh.idx[e.b + i] = sh.tmp[e.b + i];
+    const int id = slot_base + 2 * (e.b + nl - 1);
+    if (lane == 0) {
+        nodes[e.node].lo.w = __int_as_float(id);
+        nodes[e.node].hi.w = __int_as_float(id + 1);
+    }
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        const float3 l = warp_min3(lo[side]), h = warp_max3(hi[side]);
+        const float3 cl = warp_min3(clo[side]), ch = warp_max3(chi[side]);
+        if (lane != 0) continue;
+        const int b = side ? e.b + nl : e.b, c = side ? e.c - nl : nl;
+        put_node(nodes, bfirst, bcount, id + side, l, h, begin + b, c, c <= max_leaf);
+        if (c <= max_leaf) continue;
+        if (c <= kTiny) {
+            const int k = atomicAdd(&sh.n_tiny, 1);
+            if (k < kSmall / 2) sh.tiny[k] = make_int2(id + side, b | c << 16);
+            else raise_err(err, kErrStackOverflow);
+        } else {
+            const int k = atomicAdd(&sh.n_list[next], 1);
+            if (k < kSbNodes) {
+                SbNode n;
+                n.node = id + side; n.b = b; n.c = c;
+                n.clo[0] = cl.x; n.clo[1] = cl.y; n.clo[2] = cl.z;
+                n.chi[0] = ch.x; n.chi[1] = ch.y; n.chi[2] = ch.z;
+                sh.list[next][k] = n;
+            } else {
+                raise_err(err, kErrStackOverflow);
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kSbThreads, 2) k_small_build(const Task *tasks, const int *slot_bases, int ntasks,
+                                                               const float4 *__restrict__ plo,
+                                                               const float4 *__restrict__ phi, int *ref,
+                                                               BinNode *nodes, int *bfirst, int *bcount, int cap,
+                                                               int max_leaf, int *err) {
+    extern __shared__ __align__(16) unsigned char sb_raw[];
+    SbShared &sh = *reinterpret_cast<SbShared *>(sb_raw);
+    if (blockIdx.x >= ntasks) return;
+    const Task tk = tasks[blockIdx.x];
+    const int m = tk.count, slot_base = slot_bases[blockIdx.x];
+    if (m > kSmall || m < 1 || tk.node < 0 || tk.node >= cap || slot_base < 0 || slot_base + 2 * (m - 1) > cap) {
+        if (threadIdx.x == 0) raise_err(err, m > kSmall || m < 1 ? kErrSmallTooBig : kErrNodeOverflow);
+        return;
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i < m; i += kSbThreads) {
+        const int p = ref[tk.begin + i];
+        const float4 l = plo[p], h = phi[p];
+        sh.prim[i] = p;
+        sh.idx[i] = (unsigned short)i;
+        sh.box[0][i] = l.x; sh.box[1][i] = l.y; sh.box[2][i] = l.z;
+        sh.box[3][i] = h.x; sh.box[4][i] = h.y; sh.box[5][i] = h.z;
+    }
     if (threadIdx.x == 0) {
-        SmallEntry e;
-        e.node = tk.node; e.b = 0; e.c = m;
-        for (int a = 0; a < 3; ++a) { e.clo[a] = tk.clo[a]; e.chi[a] = tk.chi[a]; }
-        stack[0] = e;
-        sp = 1;
-        next_slot = slot_base[t];
+        sh.n_list[0] = sh.n_list[1] = sh.n_tiny = 0;
+        bfirst[tk.node] = tk.begin;
+        bcount[tk.node] = m;
+        if (m <= max_leaf) {
+            nodes[tk.node].lo.w = __int_as_float(tk.begin);
+            nodes[tk.node].hi.w = __int_as_float(-m);
+        } else if (m <= kTiny) {
+            sh.tiny[0] = make_int2(tk.node, m << 16);
+            sh.n_tiny = 1;
+        } else {
+            SbNode n;
+            n.node = tk.node; n.b = 0; n.c = m;
+            for (int a = 0; a < 3; ++a) { n.clo[a] = tk.clo[a]; n.chi[a] = tk.chi[a]; }
+            sh.list[0][0] = n;
+            sh.n_list[0] = 1;
+        }
     }
     __syncthreads();
-    const int my_end = slot_end[t];
-    __shared__ int stop;
-    while (true) {
-        __syncthreads();
-        const int sp_now = sp;
-        __syncthreads();
-        if (sp_now == 0) break;
-        if (threadIdx.x == 0) cur = stack[--sp];
-        __syncthreads();
-        const SmallEntry e = cur;
-        if (e.node < 0 || e.node >= cap) {  // uniform: every thread reads the same `cur`
-            if (threadIdx.x == 0) raise_err(err, kErrNodeOverflow);
-            break;
-        }
-        if (threadIdx.x == 0) {
-            bfirst[e.node] = tk.begin + e.b;
-            bcount[e.node] = e.c;
-        }
-        if (e.c <= max_leaf) {
-            if (threadIdx.x == 0) {
-                nodes[e.node].lo.w = __int_as_float(tk.begin + e.b);
-                nodes[e.node].hi.w = __int_as_float(-e.c);
-            }
-            continue;
-        }
-        // bin
-        float sc[3];
-        for (int a = 0; a < 3; ++a) sc[a] = bin_scale(e.clo[a], e.chi[a]);
-        init_bins(bins);
-        __syncthreads();
-        for (int i = threadIdx.x; i < e.c; i += blockDim.x) {
-            int p = sref[e.b + i];
-            float4 lo = plo[p], hi = phi[p];
-            bin_prim(bins, lo, hi, centroid(lo, hi), e.clo, sc, false);
-        }
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            WarpSplit w = warp_best_split(bins);
-            if (threadIdx.x == 0) best = w;
-        }
-        __syncthreads();
-        const WarpSplit bs = best;
-        // stable partition of sref[e.b .. e.b+c)
-        int lefts = 0;
-        for (int base = 0; base < e.c; base += blockDim.x) {
-            int i = base + threadIdx.x;
-            bool valid = i < e.c;
-            int p = valid ? sref[e.b + i] : 0;
-            bool l = false;
-            if (valid) {
-                if (bs.axis < 0) l = i < e.c / 2;
-                else {
-                    float3 c = centroid(plo[p], phi[p]);
-                    l = bin_of(comp(c, bs.axis), e.clo[bs.axis], sc[bs.axis]) <= bs.bin;
+    for (int cur = 0;; cur ^= 1) {
+        const int n = min(sh.n_list[cur], kSbNodes);  // uniform: last written before a barrier
+        if (n == 0) break;
+        const int wpn = max(1, kSbWarps / n), groups = kSbWarps / wpn;
+        const int g = warp / wpn, wi = warp % wpn;
+        for (int base = 0; base < n; base += groups) {
+            const bool act = g < groups && base + g < n;
+            int *bins = sh.bins[g < groups ? g : 0];
+            if (act)
+                for (int i = wi * 32 + lane; i < kSbBins; i += wpn * 32) {
+                    const int k = i % kSbBinInts;
+                    bins[i] = k == 0 ? 0 : (k <= 3 ? f2o(INFINITY) : f2o(-INFINITY));
                 }
-            }
-            int tot;
-            int rank = block_excl_scan(l ? 1 : 0, ws, &tot);
-            if (valid && l) stmp[lefts + rank] = p;
-            lefts += tot;
-        }
-        __syncthreads();
-        int nl = lefts;
-        int rights = 0;
-        for (int base = 0; base < e.c; base += blockDim.x) {
-            int i = base + threadIdx.x;
-            bool valid = i < e.c;
-            int p = valid ? sref[e.b + i] : 0;
-            bool r = false;
-            if (valid) {
-                if (bs.axis < 0) r = !(i < e.c / 2);
-                else {
-                    float3 c = centroid(plo[p], phi[p]);
-                    r = !(bin_of(comp(c, bs.axis), e.clo[bs.axis], sc[bs.axis]) <= bs.bin);
-                }
-            }
-            int tot;
-            int rank = block_excl_scan(r ? 1 : 0, ws, &tot);
-            if (valid && r) stmp[nl + rights + rank] = p;
-            rights += tot;
-        }
-        __syncthreads();
-        if (nl == 0 || nl == e.c) nl = e.c / 2;  // cannot happen with a valid plane; keep the tree finite
-        for (int i = threadIdx.x; i < e.c; i += blockDim.x) sref[e.b + i] = stmp[i];
-        __syncthreads();
-        // exact child boxes and centroid bounds by reduction
-        for (int side = 0; side < 2; ++side) {
-            int b0 = side == 0 ? 0 : nl, b1 = side == 0 ? nl : e.c;
-            float3 lo = f3(INFINITY, INFINITY, INFINITY), hi = f3(-INFINITY, -INFINITY, -INFINITY);
-            float3 clo = lo, chi = hi;
-            for (int i = b0 + threadIdx.x; i < b1; i += blockDim.x) {
-                int p = sref[e.b + i];
-                float4 l4 = plo[p], h4 = phi[p];
-                lo = fmin3(lo, f3(l4)); hi = fmax3(hi, f3(h4));
-                float3 c = centroid(l4, h4);
-                clo = fmin3(clo, c); chi = fmax3(chi, c);
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                lo = fmin3(lo, f3(__shfl_xor_sync(~0u, lo.x, o), __shfl_xor_sync(~0u, lo.y, o), __shfl_xor_sync(~0u, lo.z, o)));
-                hi = fmax3(hi, f3(__shfl_xor_sync(~0u, hi.x, o), __shfl_xor_sync(~0u, hi.y, o), __shfl_xor_sync(~0u, hi.z, o)));
-                clo = fmin3(clo, f3(__shfl_xor_sync(~0u, clo.x, o), __shfl_xor_sync(~0u, clo.y, o), __shfl_xor_sync(~0u, clo.z, o)));
-                chi = fmax3(chi, f3(__shfl_xor_sync(~0u, chi.x, o), __shfl_xor_sync(~0u, chi.y, o), __shfl_xor_sync(~0u, chi.z, o)));
-            }
-            const int w = threadIdx.x >> 5;
-            if ((threadIdx.x & 31) == 0) {
-                red[w][0] = lo.x; red[w][1] = lo.y; red[w][2] = lo.z;
-                red[w][3] = hi.x; red[w][4] = hi.y; red[w][5] = hi.z;
-                red[w][6] = clo.x; red[w][7] = clo.y; red[w][8] = clo.z;
-                red[w][9] = chi.x; red[w][10] = chi.y; red[w][11] = chi.z;
-            }
             __syncthreads();
-            if (threadIdx.x == 0) {
-                float r[12];
-                for (int k = 0; k < 12; ++k) r[k] = red[0][k];
-                for (int ww = 1; ww < kThreads / 32; ++ww)
-                    for (int k = 0; k < 12; ++k)
-                        r[k] = (k < 3 || (k >= 6 && k < 9)) ? fminf(r[k], red[ww][k]) : fmaxf(r[k], red[ww][k]);
-                int id = next_slot + side;
-                if (id >= my_end || id >= cap) {
-                    raise_err(err, kErrNodeOverflow);
-                } else {
-                    BinNode nd;
-                    nd.lo = make_float4(r[0], r[1], r[2], 0.0f);
-                    nd.hi = make_float4(r[3], r[4], r[5], 0.0f);
-                    nodes[id] = nd;
-                    SmallEntry ce;
-                    ce.node = id;
-                    ce.b = e.b + b0;
-                    ce.c = b1 - b0;
-                    for (int a = 0; a < 3; ++a) { ce.clo[a] = r[6 + a]; ce.chi[a] = r[9 + a]; }
-                    if (side == 0) cur = ce;
-                    else {
-                        // push larger first, then smaller (smaller is processed next)
-                        SmallEntry le = cur;
-                        SmallEntry big = le.c >= ce.c ? le : ce;
-                        SmallEntry small = le.c >= ce.c ? ce : le;
-                        if (sp + 2 > kStack) {
-                            raise_err(err, kErrStackOverflow);
-                        } else {
-                            stack[sp++] = big;
-                            stack[sp++] = small;
-                        }
-                        nodes[e.node].lo.w = __int_as_float(le.node);
-                        nodes[e.node].hi.w = __int_as_float(ce.node);
+            if (act) {
+                const SbNode e = sh.list[cur][base + g];
+                float sc[3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) sc[a] = bin_scale(e.clo[a], e.chi[a]);
+                for (int i = wi * 32 + lane; i < e.c; i += wpn * 32) {
+                    const int local = sh.idx[e.b + i];
+                    float3 l = f3(sh.box[0][local], sh.box[1][local], sh.box[2][local]);
+                    float3 h = f3(sh.box[3][local], sh.box[4][local], sh.box[5][local]);
+                    const float3 c = f3(0.5f * (l.x + h.x), 0.5f * (l.y + h.y), 0.5f * (l.z + h.z));
+                    const int o[6] = {f2o(l.x), f2o(l.y), f2o(l.z), f2o(h.x), f2o(h.y), f2o(h.z)};
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        int *B = bins + (a * kBins + bin_of(comp(c, a), e.clo[a], sc[a])) * kSbBinInts;
+                        atomicAdd(&B[0], 1);
+                        atomicMin(&B[1], o[0]); atomicMin(&B[2], o[1]); atomicMin(&B[3], o[2]);
+                        atomicMax(&B[4], o[3]); atomicMax(&B[5], o[4]); atomicMax(&B[6], o[5]);
                     }
                 }
             }
             __syncthreads();
+            if (act && wi == 0)
+                sb_split(sh, sh.list[cur][base + g], bins, cur ^ 1, tk.begin, slot_base, max_leaf, nodes, bfirst,
+                         bcount, err);
+            __syncthreads();
         }
-        if (threadIdx.x == 0) {
-            next_slot += 2;
-            stop = *((volatile int *)err);
-        }
+        if (threadIdx.x == 0) sh.n_list[cur] = 0;
         __syncthreads();
-        if (stop != 0) break;
+    }
+    const int nt = min(sh.n_tiny, kSmall / 2);
+    for (int k = warp; k < nt; k += kSbWarps) {
+        const int2 e = sh.tiny[k];
+        tiny_build(sh, e.x, e.y & 0xffff, e.y >> 16, tk.begin, slot_base, max_leaf, nodes, bfirst, bcount);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < m; i += blockDim.x) ref[tk.begin + i] = sref[i];
+    for (int i = threadIdx.x; i < m; i += kSbThreads) ref[tk.begin + i] = sh.prim[sh.idx[i]];
 }
 
 // ---------------------------------------------------------------------------
@@ -1094,13 +1288,11 @@ kgk_status bvh_build(DevScene &s, cudaStream_t st, BvhBuildStats *out) {
             const Split &s2 = sp[t];
             const int l = node_counter, r = node_counter + 1;
             node_counter += 2;
-            // parent's child links
-            int pi = -1;
-            for (int k = (int)h_ids.size() - 1; k >= 0; --k)
-                if (h_ids[k] == tk.node) { pi = k; break; }
-            if (pi < 0) return fail(KGK_ERR_DEVICE_CHECK, "bvh_build: lost a parent node");
-            h_vals[pi].lo.w = host_f(l);
-            h_vals[pi].hi.w = host_f(r);
+            // parent's child links (ids are handed out in order: an id is its place in the list)
+            if (tk.node >= (int)h_ids.size() || h_ids[tk.node] != tk.node)
+                return fail(KGK_ERR_DEVICE_CHECK, "bvh_build: lost a parent node");
+            h_vals[tk.node].lo.w = host_f(l);
+            h_vals[tk.node].hi.w = host_f(r);
             for (int side = 0; side < 2; ++side) {
                 Task c{};
                 c.node = side == 0 ? l : r;
@@ -1137,25 +1329,24 @@ kgk_status bvh_build(DevScene &s, cudaStream_t st, BvhBuildStats *out) {
     // small subtrees: each task of m primitives owns 2m-2 node slots
     if (!small.empty()) {
         const int ns = (int)small.size();
-        std::vector<int> sb(ns), se(ns);
+        std::vector<int> sb(ns);
         long long next = node_counter;
         for (int t = 0; t < ns; ++t) {
             sb[t] = (int)next;
             next += 2LL * small[t].count - 2;
-            se[t] = (int)next;
         }
         if (next > cap) return fail(KGK_ERR_DEVICE_CHECK, "bvh_build: node budget exceeded");
         node_counter = (int)next;
         Task *d_small;
-        int *d_sb, *d_se;
+        int *d_sb;
         KGK_TRY(buf.get(&d_small, ns, "bvh small tasks"));
         KGK_TRY(buf.get(&d_sb, ns, "bvh small tasks"));
-        KGK_TRY(buf.get(&d_se, ns, "bvh small tasks"));
         KGK_CUDA(cudaMemcpyAsync(d_small, small.data(), sizeof(Task) * ns, cudaMemcpyHostToDevice, st));
         KGK_CUDA(cudaMemcpyAsync(d_sb, sb.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, st));
-        KGK_CUDA(cudaMemcpyAsync(d_se, se.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, st));
-        k_small_build<<<ns, kThreads, 0, st>>>(d_small, d_sb, d_se, ns, plo, phi, ref, nodes, bfirst,
-                                               bcount, cap, max_leaf, err);
+        KGK_CUDA(cudaFuncSetAttribute(k_small_build, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(SbShared)));
+        k_small_build<<<ns, kSbThreads, sizeof(SbShared), st>>>(d_small, d_sb, ns, plo, phi, ref, nodes, bfirst,
+                                                                bcount, cap, max_leaf, err);
         KGK_CUDA(cudaGetLastError());
     }
     int herr = 0;
