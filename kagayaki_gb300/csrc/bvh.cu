@@ -1010,14 +1010,13 @@ __global__ void k_collapse_emit(const int *tasks, int ntasks, const int *child_l
     float3 ext = (phi - plo) * (1.0f + 1.0f / 1048576.0f);
     int ex = quant_exponent(ext.x), ey = quant_exponent(ext.y), ez = quant_exponent(ext.z);
     float sx = ldexpf(1.0f, ex - 127), sy = ldexpf(1.0f, ey - 127), sz = ldexpf(1.0f, ez - 127);
-    unsigned meta[8], qlx[8], qly[8], qlz[8], qhx[8], qhy[8], qhz[8];
-    unsigned imask = 0;
+    unsigned qlx[8], qly[8], qlz[8], qhx[8], qhy[8], qhz[8];
+    unsigned imask = 0, leaves = 0;
     const int child_base = next_start + inner_scan[t];
     const int tri_base = tri_start + tri_scan[t];
     int inner_k = 0, tri_off = 0;
     for (int s = 0; s < 8; ++s) {
         int i = child_in_slot[s];
-        meta[s] = 0;
         qlx[s] = qly[s] = qlz[s] = 0;
         qhx[s] = qhy[s] = qhz[s] = 0;
         if (i < 0) continue;
@@ -1036,27 +1035,26 @@ __global__ void k_collapse_emit(const int *tasks, int ntasks, const int *child_l
             int pos = inner_scan[t] + inner_k;
             if (pos >= next_cap || wid >= wide_cap) { raise_err(err, kErrWideOverflow); return; }
             next_tasks[pos] = c;
-            meta[s] = 0x20u | (unsigned)(24 + s);
             imask |= 1u << s;
             ++inner_k;
         } else {
-            if (tri_off + k > 24 || tri_base + tri_off + k > n_tris) { raise_err(err, kErrTriOverflow); return; }
-            unsigned unary = k == 1 ? 1u : (k == 2 ? 3u : 7u);
-            meta[s] = (unary << 5) | (unsigned)tri_off;
-            int f = bfirst[c];
-            if (f < 0 || f + k > n_tris) { raise_err(err, kErrTriOverflow); return; }
-            for (int j = 0; j < k; ++j) {
-                int prim = ref[f + j];
-                if (prim < 0 || prim >= n_tris) { raise_err(err, kErrTriOverflow); return; }
-                int dst = tri_base + tri_off + j;
-                float4 a = verts[3 * prim], b = verts[3 * prim + 1], cc = verts[3 * prim + 2];
-                tri_rec[3 * dst] = make_float4(a.x, a.y, a.z, __int_as_float(prim));
-                tri_rec[3 * dst + 1] = make_float4(b.x, b.y, b.z, 0.0f);
-                tri_rec[3 * dst + 2] = make_float4(cc.x, cc.y, cc.z, 0.0f);
-            }
-            tri_off += k;
+            if (k < 1 || k > kMaxLeaf) { raise_err(err, kErrTriOverflow); return; }
+            for (int j = 0; j < k; ++j) leaves |= 1u << (s + 8 * j);
         }
     }
+    // triangles in the order of their bits: every leaf's first, then the second ones, ...
+    for (int j = 0; j < kMaxLeaf; ++j)
+        for (int s = 0; s < 8; ++s) {
+            if (!((leaves >> (s + 8 * j)) & 1u)) continue;
+            const int f = bfirst[C[child_in_slot[s]]] + j, dst = tri_base + tri_off++;
+            if (f < 0 || f >= n_tris || dst >= n_tris) { raise_err(err, kErrTriOverflow); return; }
+            const int prim = ref[f];
+            if (prim < 0 || prim >= n_tris) { raise_err(err, kErrTriOverflow); return; }
+            const float4 a = verts[3 * prim], b = verts[3 * prim + 1], cc = verts[3 * prim + 2];
+            tri_rec[3 * dst] = make_float4(a.x, a.y, a.z, __int_as_float(prim));
+            tri_rec[3 * dst + 1] = make_float4(b.x, b.y, b.z, 0.0f);
+            tri_rec[3 * dst + 2] = make_float4(cc.x, cc.y, cc.z, 0.0f);
+        }
     int me = level_start + t;
     if (me >= wide_cap) { raise_err(err, kErrWideOverflow); return; }
     auto pack4 = [](const unsigned *v, int o) {
@@ -1064,9 +1062,9 @@ __global__ void k_collapse_emit(const int *tasks, int ntasks, const int *child_l
     };
     WideNode w;
     w.n0 = make_float4(plo.x, plo.y, plo.z,
-                       __uint_as_float((unsigned)ex | ((unsigned)ey << 8) | ((unsigned)ez << 16) | (imask << 24)));
+                       __uint_as_float((unsigned)ex | ((unsigned)ey << 8) | ((unsigned)ez << 16)));
     w.n1 = make_float4(__int_as_float(child_base), __int_as_float(tri_base),
-                       __uint_as_float(pack4(meta, 0)), __uint_as_float(pack4(meta, 4)));
+                       __uint_as_float(leaves | imask << 24), 0.0f);
     w.n2 = make_float4(__uint_as_float(pack4(qlx, 0)), __uint_as_float(pack4(qlx, 4)),
                        __uint_as_float(pack4(qhx, 0)), __uint_as_float(pack4(qhx, 4)));
     w.n3 = make_float4(__uint_as_float(pack4(qly, 0)), __uint_as_float(pack4(qly, 4)),
@@ -1484,34 +1482,31 @@ kgk_status bvh_validate(const DevScene &s, cudaStream_t st) {
         unsigned e = u(w.n0.w);
         float sc[3];
         for (int a = 0; a < 3; ++a) sc[a] = ldexpf(1.0f, (int)byte(e, a) - 127);
-        unsigned imask = byte(e, 3);
+        const unsigned field = u(w.n1.z), imask = byte(field, 3);
         int child_base = (int)u(w.n1.x), tri_base = (int)u(w.n1.y);
-        unsigned meta_w[2] = {u(w.n1.z), u(w.n1.w)};
         unsigned ql[3][2] = {{u(w.n2.x), u(w.n2.y)}, {u(w.n3.x), u(w.n3.y)}, {u(w.n4.x), u(w.n4.y)}};
         unsigned qh[3][2] = {{u(w.n2.z), u(w.n2.w)}, {u(w.n3.z), u(w.n3.w)}, {u(w.n4.z), u(w.n4.w)}};
         int inner_k = 0;
         for (int sl = 0; sl < 8; ++sl) {
-            unsigned meta = byte(meta_w[sl / 4], sl % 4);
-            if (meta == 0) continue;
+            const bool inner = (imask >> sl) & 1u;
+            const unsigned b0 = (field >> sl) & 1u, b1 = (field >> (sl + 8)) & 1u, b2 = (field >> (sl + 16)) & 1u;
+            if (b1 > b0 || b2 > b1 || (inner && b0)) return fail(KGK_ERR_DEVICE_CHECK, "bvh_validate: bad leaf bits");
+            if (!inner && !b0) continue;
             float lo[3], hi[3];
             for (int a = 0; a < 3; ++a) {
                 lo[a] = p[a] + (float)byte(ql[a][sl / 4], sl % 4) * sc[a];
                 hi[a] = p[a] + (float)byte(qh[a][sl / 4], sl % 4) * sc[a];
                 if (lo[a] > hi[a]) return fail(KGK_ERR_DEVICE_CHECK, "bvh_validate: inverted child box");
             }
-            if ((meta & 0x1f) >= 24) {
-                if (!(imask & (1u << sl)) || (meta & 0x1f) != 24u + sl)
-                    return fail(KGK_ERR_DEVICE_CHECK, "bvh_validate: inner meta inconsistent");
+            if (inner) {
                 Item c;
                 c.node = child_base + inner_k++;
                 for (int a = 0; a < 3; ++a) { c.lo[a] = lo[a]; c.hi[a] = hi[a]; }
                 stack.push_back(c);
             } else {
-                unsigned unary = meta >> 5;
-                int k = unary == 1 ? 1 : (unary == 3 ? 2 : (unary == 7 ? 3 : 0));
-                if (k == 0) return fail(KGK_ERR_DEVICE_CHECK, "bvh_validate: bad leaf meta");
+                const int k = (int)(b0 + b1 + b2);
                 for (int j = 0; j < k; ++j) {
-                    int ti = tri_base + (int)(meta & 0x1f) + j;
+                    int ti = tri_base + __builtin_popcount(field & ((1u << (sl + 8 * j)) - 1u));
                     if (ti < 0 || ti >= n) return fail(KGK_ERR_DEVICE_CHECK, "bvh_validate: triangle index out of range");
                     int id;
                     memcpy(&id, &tri[3 * (size_t)ti].w, 4);

@@ -32,14 +32,16 @@ constexpr float kBigT = 1e38f;  // bINF, global_values.cuh:10
 
 // ---------------------------------------------------------------------------
 // Compressed 8-wide BVH node (80 B = 5 x 16 B, read as five float4):
-//   n0 = (p.x, p.y, p.z, e_x | e_y << 8 | e_z << 16 | imask << 24)
-//   n1 = (child_base, tri_base, meta[0..3], meta[4..7])
+//   n0 = (p.x, p.y, p.z, e_x | e_y << 8 | e_z << 16)
+//   n1 = (child_base, tri_base, leaves | imask << 24, unused)
 //   n2 = (qlo_x[0..3], qlo_x[4..7], qhi_x[0..3], qhi_x[4..7])
 //   n3 = same for y, n4 = same for z
-// Child box a-extent = p.a + q * 2^(e_a - 127).  meta per slot: 0 = empty;
-// inner child = 0x20 | (24 + slot) (inner children are stored contiguously
-// from child_base in slot order); leaf child = (unary triangle count 1..3) << 5
-// | offset of its first triangle from tri_base.
+// Child box a-extent = p.a + q * 2^(e_a - 127).  imask: the slots that hold
+// inner children, stored contiguously from child_base in slot order.  leaves:
+// bit s + 8 j is set when slot s is a leaf with more than j triangles (1..3);
+// the node's triangles lie from tri_base in the order of their bits, so the
+// triangle of bit b is tri_base + popc(leaves & ((1 << b) - 1)), and the hit
+// mask of eight slots times 0x010101 selects the triangles of the hit leaves.
 // ---------------------------------------------------------------------------
 struct __align__(16) WideNode {
     float4 n0, n1, n2, n3, n4;

@@ -352,8 +352,9 @@ __global__ void __launch_bounds__(128, 8) k_extend(Params P, int cnt_idx, int de
     bool active = false, exhausted = false;
     int p = 0;
     unsigned rays = 0;
-    RayPre r;
-    Trav c;
+    __shared__ WarpRays s_w[4];
+    WarpRays &w = s_w[threadIdx.x >> 5];
+    Lane c;
     TravStack stk;
     TravStats st{0, 0, 0};
     while (true) {
@@ -368,21 +369,22 @@ __global__ void __launch_bounds__(128, 8) k_extend(Params P, int cnt_idx, int de
                 if (i < n) {
                     p = i;
                     const float4 o = P.cur.o[p], d = P.cur.d[p];
-                    r = make_ray(f3(o), f3(d));
-                    trav_init(c, kBigT);
+                    lane_init(w, c, f3(o), f3(d), kBigT, false);
                     active = true;
                 }
             }
         }
         if (!__any_sync(~0u, active)) break;
         int cls = -1;
-        if (active && trav_step<kCount>(s.nodes, (unsigned)s.n_nodes, s.tri_rec, (unsigned)s.n_tris, r, c, stk,
-                                        false, st)) {
+        if (warp_step<kCount>(s.nodes, (unsigned)s.n_nodes, s.tri_rec, (unsigned)s.n_tris, w, c, stk, active, false,
+                              st)) {
             active = false;
             ++rays;
-            cls = c.hit_slot < 0 ? 0 : 1 + (c.hit_slot & 1);
-            P.hit[p] = c.hit_slot < 0 ? make_float4(kBigT, 0.0f, 0.0f, __int_as_float(-1))
-                                      : make_float4(c.best_t, c.bu, c.bv, __int_as_float(c.best_id));
+            const int hs = w.slot[lane];
+            const float2 uv = w.uv[lane];
+            cls = hs < 0 ? 0 : 1 + (hs & 1);
+            P.hit[p] = hs < 0 ? make_float4(kBigT, 0.0f, 0.0f, __int_as_float(-1))
+                              : make_float4(c.best_t, uv.x, uv.y, __int_as_float(w.id[lane]));
         }
         if (__any_sync(~0u, cls >= 0)) {
             mb.add(cls == 0, p, mq, &P.cnt[kMQ]);
@@ -1214,8 +1216,9 @@ __global__ void __launch_bounds__(128, 8) k_tail_shadow(Params P) {
     bool active = false, exhausted = false;
     int slot = 0;
     unsigned rays = 0;
-    RayPre r;
-    Trav c;
+    __shared__ WarpRays s_w[4];
+    WarpRays &w = s_w[threadIdx.x >> 5];
+    Lane c;
     TravStack stk;
     TravStats st{0, 0, 0};
     while (true) {
@@ -1230,18 +1233,17 @@ __global__ void __launch_bounds__(128, 8) k_tail_shadow(Params P) {
                 if (i < n) {
                     slot = P.td_list[i];
                     const float4 o = P.td_o[slot], d = P.td_d[slot];
-                    r = make_ray(f3(o), f3(d));
-                    trav_init(c, o.w);
+                    lane_init(w, c, f3(o), f3(d), o.w, true);
                     active = true;
                 }
             }
         }
         if (!__any_sync(~0u, active)) break;
-        if (active && trav_step<false, kNodesPerStepShadow>(s.nodes, (unsigned)s.n_nodes, s.tri_rec,
-                                                            (unsigned)s.n_tris, r, c, stk, true, st)) {
+        if (warp_step<false, kNodesPerStepShadow>(s.nodes, (unsigned)s.n_nodes, s.tri_rec, (unsigned)s.n_tris, w, c,
+                                                  stk, active, true, st)) {
             active = false;
             ++rays;
-            P.td_vis[slot] = c.hit_slot < 0 ? 1 : 0;
+            P.td_vis[slot] = w.slot[lane] < 0 ? 1 : 0;
         }
     }
     warp_add_u64(&P.stats[kRaysS], rays);
@@ -1291,8 +1293,9 @@ __global__ void __launch_bounds__(128, 8) k_shadow(Params P, int cidx, int fidx,
     bool active = false, exhausted = false;
     int i = 0, light = -1;
     unsigned rays = 0;
-    RayPre r;
-    Trav c;
+    __shared__ WarpRays s_w[4];
+    WarpRays &w = s_w[threadIdx.x >> 5];
+    Lane c;
     TravStack stk;
     TravStats st{0, 0, 0};
     while (true) {
@@ -1306,19 +1309,18 @@ __global__ void __launch_bounds__(128, 8) k_shadow(Params P, int cidx, int fidx,
                 i = base + __popc(idle & lt);
                 if (i < n) {
                     const float4 o = so[i], d = sd[i];
-                    r = make_ray(f3(o), f3(d));
                     light = __float_as_int(d.w);
-                    trav_init(c, o.w);
+                    lane_init(w, c, f3(o), f3(d), o.w, light < 0);
                     active = true;
                 }
             }
         }
         if (!__any_sync(~0u, active)) break;
-        if (active && trav_step<false, kNodesPerStepShadow>(s.nodes, (unsigned)s.n_nodes, s.tri_rec,
-                                                            (unsigned)s.n_tris, r, c, stk, light < 0, st)) {
+        if (warp_step<false, kNodesPerStepShadow>(s.nodes, (unsigned)s.n_nodes, s.tri_rec, (unsigned)s.n_tris, w, c,
+                                                  stk, active, light < 0, st)) {
             active = false;
             ++rays;
-            const bool vis = light >= 0 ? (c.hit_slot >= 0 && c.best_id == light) : c.hit_slot < 0;
+            const bool vis = light >= 0 ? (w.slot[lane] >= 0 && w.id[lane] == light) : w.slot[lane] < 0;
             if (vis) {
                 const float4 cc = sc[i];
                 const int t = __float_as_int(cc.w);

@@ -36,13 +36,13 @@ __device__ __forceinline__ void flush_counters(TraceCounters *ctr, unsigned node
 }
 
 // Lanes take new rays (one atomic per warp) whenever kRefill or more of them
-// are idle, so a warp does not wait for its longest ray; trav_step keeps the
+// are idle, so a warp does not wait for its longest ray; warp_step keeps the
 // same node and triangle order as trace_closest / trace_any, so the answers
 // are the same.
 constexpr int kRefill = 8;
 
 template <bool kAny, bool kCount>
-__global__ void __launch_bounds__(128) k_trace(const WideNode *__restrict__ nodes, unsigned n_nodes,
+__global__ void __launch_bounds__(128, 8) k_trace(const WideNode *__restrict__ nodes, unsigned n_nodes,
                                                const float4 *__restrict__ tri, unsigned n_tris,
                                                const kgk_ray *__restrict__ rays, const float *__restrict__ tmax,
                                                int n, int32_t *id_out, float *t_out, uint8_t *occ,
@@ -52,8 +52,9 @@ __global__ void __launch_bounds__(128) k_trace(const WideNode *__restrict__ node
     bool active = false, exhausted = false;
     int i = 0;
     unsigned done = 0;
-    RayPre r;
-    Trav c;
+    __shared__ WarpRays s_w[4];
+    WarpRays &w = s_w[threadIdx.x >> 5];
+    Lane c;
     TravStack stk;
     TravStats st{0, 0, 0};
     while (true) {
@@ -68,21 +69,21 @@ __global__ void __launch_bounds__(128) k_trace(const WideNode *__restrict__ node
                 if (i < n) {
                     float3 o, d;
                     load_ray(rays, i, o, d);
-                    r = make_ray(o, d);
-                    trav_init(c, kAny && tmax ? tmax[i] : kBigT);
+                    lane_init(w, c, o, d, kAny && tmax ? tmax[i] : kBigT, kAny);
                     active = true;
                 }
             }
         }
         if (!__any_sync(~0u, active)) break;
-        if (active && trav_step<kCount>(nodes, n_nodes, tri, n_tris, r, c, stk, kAny, st)) {
+        if (warp_step<kCount>(nodes, n_nodes, tri, n_tris, w, c, stk, active, kAny, st)) {
             active = false;
             ++done;
+            const bool hit = w.slot[lane] >= 0;
             if (kAny) {
-                occ[i] = c.hit_slot >= 0 ? 1 : 0;
+                occ[i] = hit ? 1 : 0;
             } else {
-                id_out[i] = c.hit_slot >= 0 ? c.best_id : -1;
-                t_out[i] = c.hit_slot >= 0 ? c.best_t : kBigT;
+                id_out[i] = hit ? w.id[lane] : -1;
+                t_out[i] = hit ? c.best_t : kBigT;
             }
         }
     }

@@ -23,22 +23,39 @@ constexpr int kTravStack = 32;
 // (the closest-hit rays of k_extend and the batch queries; the shadow passes).
 constexpr int kNodesPerStep = 2;
 constexpr int kNodesPerStepShadow = 2;
-// Conservative widening of box exit distances: 1 + 2 * gamma(5) covers the
-// rounding of the origin offset, the multiply, the two roundings of the
-// biased plane offset and the plane's multiply-add.
-constexpr float kBoxWiden = 1.0000006f;
+// Conservative slack of box planes relative to the node's offset (64 units of
+// 2^-24, see node_intersect), and widening of the search limit.
+constexpr float kBoxSlack = 0x1p-18f;
+constexpr float kBoxWiden = 1.0000012f;
 
 struct RayPre {
     float3 o, d, inv;
     float sx, sy, sz;
     int kx, ky, kz;
-    unsigned oct_inv4;
+    unsigned oct;  // octant_masks
 };
 
 __device__ __forceinline__ float safe_inv(float d) {
     // |d| < 1e-20 -> +-1e20 so that scale * inv never forms 0 * inf
     float a = fabsf(d) < 1e-20f ? copysignf(1e-20f, d) : d;
     return 1.0f / a;
+}
+
+// A node's children are visited by slot XOR (7 - octant), nearest first.  The
+// three masks of the delta swaps that permute eight slot bits this way (swap
+// neighbours, pairs, nibbles), a byte each; the bits themselves are those of
+// 7 - octant (bit 0, 9 and 18).
+__device__ __forceinline__ unsigned octant_masks(float3 d) {
+    return (d.z < 0.0f ? 0u : 0x55u) | (d.y < 0.0f ? 0u : 0x3300u) | (d.x < 0.0f ? 0u : 0x0f0000u);
+}
+__device__ __forceinline__ unsigned octant_xor(unsigned m) { return (m & 1u) | ((m >> 8) & 2u) | ((m >> 14) & 4u); }
+__device__ __forceinline__ unsigned octant_permute(unsigned x, unsigned m) {
+    unsigned t = ((x >> 1) ^ x) & m;  // x has eight bits: the other masks meet zeros
+    x ^= t ^ (t << 1);
+    t = ((x >> 2) ^ x) & (m >> 8);
+    x ^= t ^ (t << 2);
+    t = ((x >> 4) ^ x) & (m >> 16);
+    return x ^ t ^ (t << 4);
 }
 
 __device__ __forceinline__ RayPre make_ray(float3 o, float3 d) {
@@ -57,9 +74,8 @@ __device__ __forceinline__ RayPre make_ray(float3 o, float3 d) {
     const float dz = comp(d, kz);
     r.sx = comp(d, kx) / dz;
     r.sy = comp(d, ky) / dz;
-    r.sz = 1.0f / dz;
-    unsigned oct = (d.x < 0.0f ? 4u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 1u : 0u);
-    r.oct_inv4 = (7u - oct) * 0x01010101u;
+    r.sz = fabsf(dz) < 1e-20f ? 1.0f / dz : comp(r.inv, kz);
+    r.oct = octant_masks(d);
     return r;
 }
 
@@ -114,69 +130,78 @@ __device__ __forceinline__ void ref_distance(const RayPre &r, float4 a4, float4 
     *v = __fmul_rn(term1, rn_dot(se1, r.d));
 }
 
-__device__ __forceinline__ unsigned byte_of(unsigned x, int i) { return (x >> (i * 8)) & 0xffu; }
 // 2^15 + (byte i of x) as a float, exactly, in one byte permute: the byte
 // becomes mantissa bits 8..15 under the exponent of 2^15 (bits 0x47000000).
 // The box test folds the bias into its per-node plane offsets, so a plane
-// costs one permute and one multiply-add (no integer-to-float conversion and
-// no subtraction).
+// costs one permute and half of a paired multiply-add (no integer-to-float
+// conversion and no subtraction).
 __device__ __forceinline__ float byte_biased(unsigned x, int i) {
     return __uint_as_float(__byte_perm(x, 0x4700u, 0x5404u | ((unsigned)i << 4)));
 }
-__device__ __forceinline__ unsigned sign_extend_s8x4(unsigned x) { return ((x >> 7) & 0x01010101u) * 0xffu; }
+// (a0, a1) * b + (c0, c1) in one instruction (two FP32 multiply-adds, each
+// rounded as fmaf): a child's near and far plane of one axis.
+__device__ __forceinline__ float2 fma2(float a0, float a1, float b, float c0, float c1) {
+    float2 r;
+    asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\tmov.b64 c, {%5, %6};\n\t"
+        "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a0), "f"(a1), "f"(b), "f"(c0), "f"(c1));
+    return r;
+}
 
-// Child hit mask of one compressed node: bits 24..31 = inner children
-// (octant-permuted slots), bits 0..23 = triangles of hit leaf children.
-__device__ __forceinline__ unsigned node_intersect(const RayPre &r, float tmin, float tmax,
-                                                   const float4 n0, const float4 n1, const float4 n2,
-                                                   const float4 n3, const float4 n4) {
+// Hit mask of one compressed node: bits 24..31 = inner children
+// (octant-permuted slots), bits 0..23 = triangles of hit leaf children (bits
+// of the node's leaf field).
+__device__ __forceinline__ unsigned node_intersect(float3 o, float3 inv, unsigned oct, float tmax, const float4 n0,
+                                                   const float4 n1, const float4 n2, const float4 n3,
+                                                   const float4 n4) {
     const unsigned e = __float_as_uint(n0.w);
-    const float adx = __uint_as_float((e & 0xffu) << 23) * r.inv.x;
-    const float ady = __uint_as_float(((e >> 8) & 0xffu) << 23) * r.inv.y;
-    const float adz = __uint_as_float(((e >> 16) & 0xffu) << 23) * r.inv.z;
+    const float adx = __uint_as_float((e & 0xffu) << 23) * inv.x;
+    const float ady = __uint_as_float(((e >> 8) & 0xffu) << 23) * inv.y;
+    const float adz = __uint_as_float(((e >> 16) & 0xffu) << 23) * inv.z;
     // Plane b of an axis lies at t = (2^15 + b) * ad + (o - 2^15 * ad),
-    // formed as one multiply-add with an exact product.  The offset is
+    // formed as one multiply-add with an exact product.  With u = 2^-24, o
+    // carries 3 u |o| (origin offset, product, inverse); the offset is
     // rounded twice (o - 2^15 ad, then -/+ the slack), each time by at most
-    // 2^-24 (|o| + 2^15 |ad|) = 2^-24 |o| + 2^-9 |ad|.  A slack of 1/64 of the
-    // axis's quantum (|ad| / 64: per axis, since |ad| is huge on an axis the
-    // ray nearly parallels) moves near planes down and far planes up, four
-    // times the |ad| parts; kBoxWiden covers the |o| parts.
-    const float ox = (n0.x - r.o.x) * r.inv.x;
-    const float oy = (n0.y - r.o.y) * r.inv.y;
-    const float oz = (n0.z - r.o.z) * r.inv.z;
+    // u (|o| + 2^15 |ad|); the multiply-add by u (|o| + 255 |ad|); b ad carries
+    // 255 u |ad| of the inverse: together 6 u |o| + 2^-8 (1 + 2^-5) |ad|.  A
+    // slack of 64 u |o| + |ad| / 64 (per axis: |ad| is huge on an axis the ray
+    // nearly parallels) moves near planes down and far planes up; what is left
+    // of it covers the rounding of the hit distances themselves.
+    const float ox = (n0.x - o.x) * inv.x;
+    const float oy = (n0.y - o.y) * inv.y;
+    const float oz = (n0.z - o.z) * inv.z;
     const float bx = fmaf(-32768.0f, adx, ox), by = fmaf(-32768.0f, ady, oy), bz = fmaf(-32768.0f, adz, oz);
-    const float sx = fabsf(adx) * 0.015625f, sy = fabsf(ady) * 0.015625f, sz = fabsf(adz) * 0.015625f;
+    const float sx = fmaf(fabsf(ox), kBoxSlack, fabsf(adx) * 0.015625f);
+    const float sy = fmaf(fabsf(oy), kBoxSlack, fabsf(ady) * 0.015625f);
+    const float sz = fmaf(fabsf(oz), kBoxSlack, fabsf(adz) * 0.015625f);
     const float oxn = bx - sx, oyn = by - sy, ozn = bz - sz;
     const float oxf = bx + sx, oyf = by + sy, ozf = bz + sz;
     const float tm = tmax * kBoxWiden;
-    unsigned hits = 0;
+    unsigned miss = 0;  // slot 7 first, so that slot s ends at bit s
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        const unsigned meta4 = __float_as_uint(half ? n1.w : n1.z);
-        const unsigned is_inner4 = (meta4 & (meta4 << 1)) & 0x10101010u;
-        const unsigned inner_mask4 = sign_extend_s8x4(is_inner4 << 3);
-        const unsigned bit_index4 = (meta4 ^ (r.oct_inv4 & inner_mask4)) & 0x1f1f1f1fu;
-        const unsigned child_bits4 = (meta4 >> 5) & 0x07070707u;
+    for (int half = 1; half >= 0; --half) {
         const unsigned qlx = __float_as_uint(half ? n2.y : n2.x), qhx = __float_as_uint(half ? n2.w : n2.z);
         const unsigned qly = __float_as_uint(half ? n3.y : n3.x), qhy = __float_as_uint(half ? n3.w : n3.z);
         const unsigned qlz = __float_as_uint(half ? n4.y : n4.x), qhz = __float_as_uint(half ? n4.w : n4.z);
-        const unsigned xn = r.d.x < 0.0f ? qhx : qlx, xf = r.d.x < 0.0f ? qlx : qhx;
-        const unsigned yn = r.d.y < 0.0f ? qhy : qly, yf = r.d.y < 0.0f ? qly : qhy;
-        const unsigned zn = r.d.z < 0.0f ? qhz : qlz, zf = r.d.z < 0.0f ? qlz : qhz;
+        const unsigned xn = inv.x < 0.0f ? qhx : qlx, xf = inv.x < 0.0f ? qlx : qhx;
+        const unsigned yn = inv.y < 0.0f ? qhy : qly, yf = inv.y < 0.0f ? qly : qhy;
+        const unsigned zn = inv.z < 0.0f ? qhz : qlz, zf = inv.z < 0.0f ? qlz : qhz;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float t0x = fmaf(byte_biased(xn, j), adx, oxn);
-            const float t0y = fmaf(byte_biased(yn, j), ady, oyn);
-            const float t0z = fmaf(byte_biased(zn, j), adz, ozn);
-            const float t1x = fmaf(byte_biased(xf, j), adx, oxf);
-            const float t1y = fmaf(byte_biased(yf, j), ady, oyf);
-            const float t1z = fmaf(byte_biased(zf, j), adz, ozf);
-            const float lo = fmaxf(fmaxf(t0x, t0y), fmaxf(t0z, tmin));
-            const float hi = fminf(fminf(t1x, t1y), fminf(t1z, tm)) * kBoxWiden;
-            if (lo <= hi) hits |= byte_of(child_bits4, j) << byte_of(bit_index4, j);
+        for (int j = 3; j >= 0; --j) {
+            const float2 tx = fma2(byte_biased(xn, j), byte_biased(xf, j), adx, oxn, oxf);
+            const float2 ty = fma2(byte_biased(yn, j), byte_biased(yf, j), ady, oyn, oyf);
+            const float2 tz = fma2(byte_biased(zn, j), byte_biased(zf, j), adz, ozn, ozf);
+            const float lo = fmaxf(fmaxf(tx.x, ty.x), fmaxf(tz.x, 0.0f));
+            const float hi = fminf(fminf(tx.y, ty.y), fminf(tz.y, tm));
+            // the sign of hi - lo shifted in: one multiply-add-pipe instruction
+            // and one shift a slot, where a compare and the slot's own bits
+            // took five
+            miss = __funnelshift_l(__float_as_uint(hi - lo), miss, 1);
         }
     }
-    return hits;
+    const unsigned hit = ~miss & 0xffu, field = __float_as_uint(n1.z);
+    return (hit * 0x010101u & field & 0xffffffu) | octant_permute(hit & (field >> 24), oct) << 24;
 }
 
 struct TravStats {
@@ -196,9 +221,11 @@ __device__ __forceinline__ int trace_closest(const WideNode *__restrict__ nodes,
     uint2 stack[kTravStack];
     int sp = 0;
     int hit_slot = -1;
+    const unsigned oct = octant_xor(r.oct);
     uint2 group = make_uint2(0u, 0x80000000u);
     while (true) {
         uint2 tg = make_uint2(0u, 0u);
+        unsigned leaves = 0u;
         if (group.y & 0xff000000u) {
             const unsigned hits_imask = group.y;
             const int child_bit = 31 - __clz(hits_imask & 0xff000000u);
@@ -208,25 +235,23 @@ __device__ __forceinline__ int trace_closest(const WideNode *__restrict__ nodes,
                 if (sp < kTravStack) stack[sp++] = group;
                 else st.overflow = 1;
             }
-            const unsigned slot = (unsigned)(child_bit - 24) ^ (r.oct_inv4 & 0xffu);
+            const unsigned slot = (unsigned)(child_bit - 24) ^ oct;
             const unsigned rel = __popc(hits_imask & ~(0xffffffffu << slot));
             if (base + rel >= n_nodes) { st.overflow = 2; break; }
             const WideNode *nd = nodes + base + rel;
             const float4 n0 = __ldg(&nd->n0), n1 = __ldg(&nd->n1), n2 = __ldg(&nd->n2),
                          n3 = __ldg(&nd->n3), n4 = __ldg(&nd->n4);
             if (kCount) ++st.nodes;
-            const unsigned hm = node_intersect(r, 0.0f, best_t, n0, n1, n2, n3, n4);
-            const unsigned imask = __float_as_uint(n0.w) >> 24;
+            const unsigned hm = node_intersect(r.o, r.inv, r.oct, best_t, n0, n1, n2, n3, n4);
+            const unsigned imask = __float_as_uint(n1.z) >> 24;
+            leaves = __float_as_uint(n1.z);
             group = make_uint2(__float_as_uint(n1.x), (hm & 0xff000000u) | imask);
             tg = make_uint2(__float_as_uint(n1.y), hm & 0x00ffffffu);
-        } else {
-            tg = group;
-            group = make_uint2(0u, 0u);
         }
         while (tg.y != 0u) {
             const int k = __ffs(tg.y) - 1;
             tg.y &= tg.y - 1u;
-            const int ti = (int)tg.x + k;
+            const int ti = (int)tg.x + __popc(leaves & ((1u << k) - 1u));
             if ((unsigned)ti >= n_tris) { st.overflow = 2; tg.y = 0u; group = make_uint2(0u, 0u); sp = 0; break; }
             const float4 a = __ldg(&tri[3 * ti]), b = __ldg(&tri[3 * ti + 1]), c = __ldg(&tri[3 * ti + 2]);
             if (kCount) ++st.tris;
@@ -259,9 +284,11 @@ __device__ __forceinline__ bool trace_any(const WideNode *__restrict__ nodes, un
                                           const RayPre &r, float tmax, TravStats &st) {
     uint2 stack[kTravStack];
     int sp = 0;
+    const unsigned oct = octant_xor(r.oct);
     uint2 group = make_uint2(0u, 0x80000000u);
     while (true) {
         uint2 tg = make_uint2(0u, 0u);
+        unsigned leaves = 0u;
         if (group.y & 0xff000000u) {
             const unsigned hits_imask = group.y;
             const int child_bit = 31 - __clz(hits_imask & 0xff000000u);
@@ -271,25 +298,23 @@ __device__ __forceinline__ bool trace_any(const WideNode *__restrict__ nodes, un
                 if (sp < kTravStack) stack[sp++] = group;
                 else st.overflow = 1;
             }
-            const unsigned slot = (unsigned)(child_bit - 24) ^ (r.oct_inv4 & 0xffu);
+            const unsigned slot = (unsigned)(child_bit - 24) ^ oct;
             const unsigned rel = __popc(hits_imask & ~(0xffffffffu << slot));
             if (base + rel >= n_nodes) { st.overflow = 2; break; }
             const WideNode *nd = nodes + base + rel;
             const float4 n0 = __ldg(&nd->n0), n1 = __ldg(&nd->n1), n2 = __ldg(&nd->n2),
                          n3 = __ldg(&nd->n3), n4 = __ldg(&nd->n4);
             if (kCount) ++st.nodes;
-            const unsigned hm = node_intersect(r, 0.0f, tmax, n0, n1, n2, n3, n4);
-            const unsigned imask = __float_as_uint(n0.w) >> 24;
+            const unsigned hm = node_intersect(r.o, r.inv, r.oct, tmax, n0, n1, n2, n3, n4);
+            const unsigned imask = __float_as_uint(n1.z) >> 24;
+            leaves = __float_as_uint(n1.z);
             group = make_uint2(__float_as_uint(n1.x), (hm & 0xff000000u) | imask);
             tg = make_uint2(__float_as_uint(n1.y), hm & 0x00ffffffu);
-        } else {
-            tg = group;
-            group = make_uint2(0u, 0u);
         }
         while (tg.y != 0u) {
             const int k = __ffs(tg.y) - 1;
             tg.y &= tg.y - 1u;
-            const int ti = (int)tg.x + k;
+            const int ti = (int)tg.x + __popc(leaves & ((1u << k) - 1u));
             if ((unsigned)ti >= n_tris) { st.overflow = 2; tg.y = 0u; group = make_uint2(0u, 0u); sp = 0; break; }
             const float4 a = __ldg(&tri[3 * ti]), b = __ldg(&tri[3 * ti + 1]), c = __ldg(&tri[3 * ti + 2]);
             if (kCount) ++st.tris;
@@ -308,99 +333,184 @@ __device__ __forceinline__ bool trace_any(const WideNode *__restrict__ nodes, un
 }
 
 // ---------------------------------------------------------------------------
-// Resumable traversal, a few node visits per call, for kernels that refill
-// finished lanes with new rays (dynamic ray fetch) instead of letting a warp
-// wait for its longest ray.  Same node order, culling and hit rules as
+// Warp traversal: resumable, a few node visits per call, for kernels that
+// refill finished lanes with new rays (dynamic ray fetch) instead of letting a
+// warp wait for its longest ray.  Same node order, culling and hit rules as
 // trace_closest / trace_any, so the results are the same.
+//
+// Node visits run a ray per lane.  Triangle tests do not: a node yields none
+// on most lanes and several on a few, so a loop over each lane's own triangles
+// runs as long as the warp's longest list with a handful of lanes active.
+// Here the lanes list their (ray, triangle) pairs in shared memory and the
+// warp tests 32 pairs at a time, whichever rays they belong to, from a shared
+// copy of the rays; a ray's closest hit is kept in shared memory too, so the
+// lane's registers hold only what node visits need.
+// Instruction issue bounds it (76 % of slots on incoherent rays, DRAM below
+// 10 %).  On the 5.2M-triangle frame a step's own-triangle loop ran 2.6 times
+// at 6.9 lanes; pairs run 1.3 times at 14.2.  With the leaf field and the
+// paired multiply-adds of node_intersect, closest-hit batches (2^22 rays, 1.3M
+// triangles) 524 -> 479 us, the 64-sample 1080p frame 93.3 -> 89.6 ms, two
+// 1-sample orbit frames 6.73 -> 6.49 ms.  Measured and left out: keeping fewer
+// than 32 pairs for the next step (frame 88.1 ms, but orbit 6.58 ms), three
+// nodes a step (frame 90.2, batches 508 us), three-input min / max (batches
+// 490 us), seven blocks per SM without spills (frame 92.0 ms), 96-byte nodes
+// or 64-byte triangle records read by 32-byte loads (batches + 1.5 %).
 // ---------------------------------------------------------------------------
-// The stack lives in a separate local array (TravStack) so that the scalar
-// state stays in registers.
+constexpr int kPairsPerLane = 3;  // triangles a lane lists at a time (two ballots give its place)
+
+struct WarpRays {  // one warp's part of shared memory
+    float4 o[32];          // origin, shear x
+    float4 d[32];          // direction, shear y
+    float2 z[32];          // shear z; axes kx | ky << 2 | kz << 4, bit 8: occlusion
+    unsigned t[32];        // closest hit: distance bits (the search limit before any hit),
+    int id[32], slot[32];  // triangle, 2 * BVH-order index + material class (-1: no hit),
+    float2 uv[32];         // barycentrics
+    int2 pair[32 * kPairsPerLane];  // BVH-order triangle, owning lane
+};
+
+// What a lane keeps of its ray between steps.
+struct Lane {
+    float3 o, inv;
+    unsigned oct;       // octant_masks
+    uint2 group;
+    int sp;
+    float best_t;
+};
+// The stack lives in a separate local array so that the scalar state stays in
+// registers.
 struct TravStack {
     uint2 e[kTravStack];
 };
-struct Trav {
-    uint2 group;
-    int sp;
-    float best_t, bu, bv;
-    int best_id, hit_slot;
-};
 
-__device__ __forceinline__ void trav_init(Trav &c, float tmax) {
-    c.sp = 0;
+__device__ __forceinline__ void lane_init(WarpRays &w, Lane &c, float3 o, float3 d, float tmax, bool any_mode) {
+    const int lane = threadIdx.x & 31;
+    const RayPre r = make_ray(o, d);
+    c.o = o;
+    c.inv = r.inv;
+    c.oct = r.oct;
     c.group = make_uint2(0u, 0x80000000u);
+    c.sp = 0;
     c.best_t = tmax;
-    c.bu = 0.0f;
-    c.bv = 0.0f;
-    c.best_id = 0x7fffffff;
-    c.hit_slot = -1;
+    w.o[lane] = make_float4(o.x, o.y, o.z, r.sx);
+    w.d[lane] = make_float4(d.x, d.y, d.z, r.sy);
+    w.z[lane] = make_float2(r.sz, __int_as_float(r.kx | r.ky << 2 | r.kz << 4 | (any_mode ? 256 : 0)));
+    w.t[lane] = __float_as_uint(tmax);
+    w.id[lane] = 0x7fffffff;
+    w.slot[lane] = -1;
 }
 
-// Visits nodes until one has hit leaf triangles (at most kNodesPerStep
-// nodes), then tests those triangles: the same order as trace_closest /
-// trace_any, in fewer, more even steps.  any_mode: stop at the
-// first triangle with kTMin <= t < best_t (occlusion); otherwise keep the
-// closest hit (ties to the smaller id).  Returns true when the traversal is
-// finished; then c.hit_slot is -1 (no hit) or, for the BVH-order triangle ti
-// hit, 2 * ti + its material class (the .w of its second record: 1 = Disney).
+// One step of the warp: active lanes visit nodes until one has hit leaf
+// triangles (at most kVisits nodes), then the warp tests all of them.
+// Returns true on a lane whose ray is finished: w.slot is -1 (no hit) or
+// names the hit; an occlusion ray ends at its first triangle with
+// kTMin <= t < its limit.  All 32 lanes must call it.
 template <bool kCount, int kVisits = kNodesPerStep>
-__device__ __forceinline__ bool trav_step(const WideNode *__restrict__ nodes, unsigned n_nodes,
-                                          const float4 *__restrict__ tri, unsigned n_tris, const RayPre &r,
-                                          Trav &c, TravStack &stk, bool any_mode, TravStats &st) {
+__device__ __forceinline__ bool warp_step(const WideNode *__restrict__ nodes, unsigned n_nodes,
+                                          const float4 *__restrict__ tri, unsigned n_tris, WarpRays &w, Lane &c,
+                                          TravStack &stk, bool active, bool any_mode, TravStats &st) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
     uint2 tg = make_uint2(0u, 0u);
+    unsigned leaves = 0u;
+    bool dead = false;
+    if (active) {
 #pragma unroll 1
-    for (int visit = 0; visit < kVisits && tg.y == 0u; ++visit) {
-        if ((c.group.y & 0xff000000u) == 0u) {
-            if (c.sp == 0) break;
-            c.group = stk.e[--c.sp];
+        for (int visit = 0; visit < kVisits && tg.y == 0u; ++visit) {
+            if ((c.group.y & 0xff000000u) == 0u) {
+                if (c.sp == 0) break;
+                c.group = stk.e[--c.sp];
+            }
+            const unsigned hits_imask = c.group.y;
+            const int child_bit = 31 - __clz(hits_imask & 0xff000000u);
+            const unsigned base = c.group.x;
+            c.group.y &= ~(1u << child_bit);
+            if (c.group.y & 0xff000000u) {
+                if (c.sp < kTravStack) stk.e[c.sp++] = c.group;
+                else st.overflow = 1;
+            }
+            const unsigned slot = (unsigned)(child_bit - 24) ^ octant_xor(c.oct);
+            const unsigned rel = __popc(hits_imask & ~(0xffffffffu << slot));
+            if (base + rel >= n_nodes) { st.overflow = 2; dead = true; break; }
+            const WideNode *nd = nodes + base + rel;
+            const float4 n0 = __ldg(&nd->n0), n1 = __ldg(&nd->n1), n2 = __ldg(&nd->n2), n3 = __ldg(&nd->n3),
+                         n4 = __ldg(&nd->n4);
+            if (kCount) ++st.nodes;
+            const unsigned hm = node_intersect(c.o, c.inv, c.oct, c.best_t, n0, n1, n2, n3, n4);
+            leaves = __float_as_uint(n1.z);
+            const unsigned imask = leaves >> 24;
+            c.group = make_uint2(__float_as_uint(n1.x), (hm & 0xff000000u) | imask);
+            tg = make_uint2(__float_as_uint(n1.y), hm & 0x00ffffffu);
         }
-        const unsigned hits_imask = c.group.y;
-        const int child_bit = 31 - __clz(hits_imask & 0xff000000u);
-        const unsigned base = c.group.x;
-        c.group.y &= ~(1u << child_bit);
-        if (c.group.y & 0xff000000u) {
-            if (c.sp < kTravStack) stk.e[c.sp++] = c.group;
-            else st.overflow = 1;
-        }
-        const unsigned slot = (unsigned)(child_bit - 24) ^ (r.oct_inv4 & 0xffu);
-        const unsigned rel = __popc(hits_imask & ~(0xffffffffu << slot));
-        if (base + rel >= n_nodes) { st.overflow = 2; return true; }
-        const WideNode *nd = nodes + base + rel;
-        const float4 n0 = __ldg(&nd->n0), n1 = __ldg(&nd->n1), n2 = __ldg(&nd->n2), n3 = __ldg(&nd->n3),
-                     n4 = __ldg(&nd->n4);
-        if (kCount) ++st.nodes;
-        const unsigned hm = node_intersect(r, 0.0f, c.best_t, n0, n1, n2, n3, n4);
-        const unsigned imask = __float_as_uint(n0.w) >> 24;
-        c.group = make_uint2(__float_as_uint(n1.x), (hm & 0xff000000u) | imask);
-        tg = make_uint2(__float_as_uint(n1.y), hm & 0x00ffffffu);
     }
-    while (tg.y != 0u) {
-        const int k = __ffs(tg.y) - 1;
-        tg.y &= tg.y - 1u;
-        const int ti = (int)tg.x + k;
-        if ((unsigned)ti >= n_tris) { st.overflow = 2; return true; }
-        const float4 a = __ldg(&tri[3 * ti]), b = __ldg(&tri[3 * ti + 1]), cc = __ldg(&tri[3 * ti + 2]);
-        if (kCount) ++st.tris;
-        float t, u, v;
-        if (tri_intersect(r, a, b, cc, &t, &u, &v)) {
-            ref_distance(r, a, b, cc, &t, &u, &v);
-            if (!(t >= kTMin)) continue;
-            const int id = __float_as_int(a.w);
-            if (any_mode) {
-                if (t < c.best_t) {
-                    c.best_t = t;
-                    c.best_id = id;
-                    c.hit_slot = 2 * ti + __float_as_int(b.w);
-                    return true;
+    bool any_hit = false;
+    while (true) {
+        const int n = min(__popc(tg.y), kPairsPerLane);
+        const unsigned b0 = __ballot_sync(~0u, n & 1), b1 = __ballot_sync(~0u, n & 2);
+        if ((b0 | b1) == 0u) break;
+        const int total = __popc(b0) + 2 * __popc(b1);
+        int at = __popc(b0 & lt) + 2 * __popc(b1 & lt);
+#pragma unroll
+        for (int i = 0; i < kPairsPerLane; ++i)
+            if (i < n) {
+                w.pair[at + i] = make_int2((int)tg.x + __popc(leaves & ((tg.y & (0u - tg.y)) - 1u)), lane);
+                tg.y &= tg.y - 1u;
+            }
+        __syncwarp();
+        for (int p0 = 0; p0 < total; p0 += 32) {
+            bool hit = false;
+            int own = 0, ti = 0, id = 0, cls = 0;
+            float t = 0.0f, u = 0.0f, v = 0.0f, old = 0.0f;
+            if (p0 + lane < total) {
+                const int2 pr = w.pair[p0 + lane];
+                ti = pr.x;
+                own = pr.y;
+                if ((unsigned)ti >= n_tris) {
+                    st.overflow = 2;
+                } else {
+                    const float4 a = __ldg(&tri[3 * ti]), b = __ldg(&tri[3 * ti + 1]), cc = __ldg(&tri[3 * ti + 2]);
+                    const float4 ro = w.o[own], rd = w.d[own];
+                    const float2 rz = w.z[own];
+                    const int ax = __float_as_int(rz.y);
+                    RayPre r;
+                    r.o = f3(ro);
+                    r.d = f3(rd);
+                    r.sx = ro.w;
+                    r.sy = rd.w;
+                    r.sz = rz.x;
+                    r.kx = ax & 3;
+                    r.ky = (ax >> 2) & 3;
+                    r.kz = (ax >> 4) & 3;
+                    if (kCount) ++st.tris;
+                    if (tri_intersect(r, a, b, cc, &t, &u, &v)) {
+                        ref_distance(r, a, b, cc, &t, &u, &v);
+                        old = __uint_as_float(w.t[own]);
+                        id = __float_as_int(a.w);
+                        cls = __float_as_int(b.w);
+                        // a tie goes to the smaller id below; an occlusion ray's limit is exclusive
+                        hit = t >= kTMin && ((ax & 256) ? t < old : t <= old);
+                    }
                 }
-            } else if (t < c.best_t || (t == c.best_t && id < c.best_id)) {
-                c.best_t = t;
-                c.best_id = id;
-                c.bu = u;
-                c.bv = v;
-                c.hit_slot = 2 * ti + __float_as_int(b.w);
+            }
+            if (!__any_sync(~0u, hit)) continue;
+            any_hit = true;
+            // distances are positive: their bits order like the values
+            if (hit) atomicMin(&w.t[own], __float_as_uint(t));
+            __syncwarp();
+            hit = hit && __float_as_uint(t) == w.t[own];
+            if (hit && t < old) w.id[own] = 0x7fffffff;
+            __syncwarp();
+            if (hit) atomicMin(&w.id[own], id);
+            __syncwarp();
+            if (hit && w.id[own] == id) {
+                w.slot[own] = 2 * ti + cls;
+                w.uv[own] = make_float2(u, v);
             }
         }
+        __syncwarp();
     }
+    if (!active) return false;
+    if (any_hit) c.best_t = __uint_as_float(w.t[lane]);
+    if (dead || (any_mode && any_hit && w.slot[lane] >= 0)) return true;
     if ((c.group.y & 0xff000000u) == 0u) {
         if (c.sp == 0) return true;
         c.group = stk.e[--c.sp];
