@@ -57,6 +57,17 @@ __device__ __forceinline__ unsigned long long splitmix64(unsigned long long z) {
 }
 
 // ---------------------------------------------------------------------------
+// Library functions out of line: their range reductions are inlined at every
+// call otherwise, and instruction fetch is what holds the shading kernels.
+// In one function the compiler merges sine and cosine into one evaluation that
+// rounds some angles differently from the two apart: each use below keeps the
+// rounding it has had (the frames depend on it to the last bit).
+static __device__ __noinline__ float2 sincos_nl(float x) { return make_float2(sinf(x), cosf(x)); }
+static __device__ __noinline__ float pow_nl(float x, float y) { return powf(x, y); }
+static __device__ __noinline__ float acos_nl(float x) { return acosf(x); }
+static __device__ __noinline__ float asin_nl(float x) { return asinf(x); }
+
+// ---------------------------------------------------------------------------
 // Frames
 // ---------------------------------------------------------------------------
 // GenerateONBFromNormal (struct_Vec.cuh:81-86).
@@ -209,13 +220,17 @@ static __device__ float disney_pdf_unbiased(const DisneyParams &p, float3 in, fl
     return pdf / sw;
 }
 
-// sample_ray_cosine_weighted (LambertBRDF_sampling.cuh:10-29).
+// sample_ray_cosine_weighted (LambertBRDF_sampling.cuh:10-29).  kInline: the
+// azimuth's sine and cosine in the caller's code (the Lambert sample) or
+// merged out of line (the Disney lobes).
+template <bool kInline>
 __device__ __forceinline__ float3 sample_cos_ref(unsigned long long &s, float3 u, float3 v, float3 w) {
     const float R1 = rnd_ref(s, 0.0f, 1.0f);
     const float R2 = rnd_ref(s, 0.0f, 0.9999f);
-    const float theta = acosf(sqrtf(1.0f - R2));
+    const float2 th = sincos_nl(acos_nl(sqrtf(1.0f - R2)));
     const float phi = 2.0f * kPI * R1;
-    return normalize3(u * (sinf(theta) * cosf(phi)) + v * (sinf(theta) * sinf(phi)) + w * cosf(theta));
+    const float2 ph = kInline ? make_float2(sinf(phi), cosf(phi)) : sincos_nl(phi);
+    return normalize3(u * (th.x * ph.y) + v * (th.x * ph.x) + w * th.y);
 }
 
 __device__ __forceinline__ float3 sample_cos_u(float r1, float r2, float3 u, float3 v, float3 w) {
@@ -226,20 +241,27 @@ __device__ __forceinline__ float3 sample_cos_u(float r1, float r2, float3 u, flo
 __device__ __forceinline__ float3 reflect_ref(float3 d, float3 h) { return normalize3(d - h * (2.0f * dot3(d, h))); }
 
 // GTR2 anisotropic half vector (Disney_BRDF_sampling.cuh:4-9) from r1, r2.
+// kInline: the library functions in the caller's code (the unbiased estimator)
+// or out of line (compat).
+template <bool kInline>
 __device__ __forceinline__ float3 gtr2_half(float R1, float R2, float3 u, float3 v, float3 w, float ax, float ay) {
-    const float3 a = u * (ax * cosf(2.0f * kPI * R1)) + v * (ay * sinf(2.0f * kPI * R1));
+    const float phi = 2.0f * kPI * R1;
+    const float2 ph = kInline ? make_float2(sinf(phi), cosf(phi)) : sincos_nl(phi);
+    const float3 a = u * (ax * ph.y) + v * (ay * ph.x);
     return normalize3(a * sqrtf(R2 / (1.0f - R2)) + w);
 }
 
 // GTR1 half vector.  The reference takes sin(phi) = +sqrt(1 - cos^2(phi))
-// (Disney_BRDF_sampling.cuh:23-30); `full_circle` restores the sign.
-__device__ __forceinline__ float3 gtr1_half(float R1, float R2, float3 u, float3 v, float3 w, float alpha,
-                                            bool full_circle) {
-    const float cphi = cosf(2.0f * kPI * R1);
-    float sphi = sqrtf(fmaxf(0.0f, 1.0f - cphi * cphi));
-    if (full_circle) sphi = sinf(2.0f * kPI * R1);
+// (Disney_BRDF_sampling.cuh:23-30); the unbiased estimator (kInline) restores
+// the sign.
+template <bool kInline>
+__device__ __forceinline__ float3 gtr1_half(float R1, float R2, float3 u, float3 v, float3 w, float alpha) {
+    const float2 ph = sincos_nl(2.0f * kPI * R1);
+    const float cphi = ph.y;
+    const float sphi = kInline ? ph.x : sqrtf(fmaxf(0.0f, 1.0f - cphi * cphi));
     alpha = fminf(fmaxf(alpha, -0.9999f), 0.9999f);
-    const float ct = sqrtf((1.0f - powf(alpha, 2.0f * (1.0f - R2))) / (1.0f - alpha * alpha));
+    const float pw = kInline ? powf(alpha, 2.0f * (1.0f - R2)) : pow_nl(alpha, 2.0f * (1.0f - R2));
+    const float ct = sqrtf((1.0f - pw) / (1.0f - alpha * alpha));
     const float st = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
     return u * (st * cphi) + v * (st * sphi) + w * ct;
 }
@@ -271,11 +293,11 @@ __device__ __forceinline__ int cdf_search(const float *c, int n, float u) {
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float2 uv_sphere_ref(float3 d) {
     float theta;
-    const float phi = asinf(d.z);
+    const float phi = asin_nl(d.z);
     if ((double)fabsf(d.z) >= 1.0 - (double)kSINF) theta = 0.0f;
     else if (fabsf(d.x) <= kSINF) theta = d.y > 0.0f ? kPI / 2 : -kPI / 2;
     else {
-        const float s = asinf(d.y / sqrtf(1.0f - d.z * d.z));
+        const float s = asin_nl(d.y / sqrtf(1.0f - d.z * d.z));
         if (d.x > 0.0f) theta = s;
         else if (d.x < 0.0f && d.y > 0.0f) theta = kPI - s;
         else theta = -1.0f * kPI - s;
@@ -315,11 +337,12 @@ __device__ __forceinline__ float3 env_index_to_dir_ref(const DevScene &s, int in
     const float v = 1.0f - (float)(index / s.env_w) / (float)s.env_h;
     const float theta = (u - 0.5f) * 2.0f * kPI;
     const float phi = (v - 0.5f) * kPI;
-    const float cp = cosf(phi);
+    const float2 th = sincos_nl(theta), ph = sincos_nl(phi);
+    const float cp = ph.y;
     if (fabsf(cp) < kSINF) pdf *= 1.0f / (2.0f * kPI * kPI * kSINF);
     else pdf *= 1.0f / (2.0f * kPI * kPI * cp);
     pdf *= (float)(s.env_w * s.env_h);
-    return f3(cp * cosf(theta), cp * sinf(theta), sinf(phi));
+    return f3(cp * th.y, cp * th.x, ph.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -375,8 +398,9 @@ __device__ __forceinline__ float3 env_sample_u(const DevScene &s, unsigned long 
     const float v = 1.0f - (row + r2) / s.env_h;
     const float u = 1.0f - (col + r3) / s.env_w;
     const float phi = (v - 0.5f) * kPI, theta = (u - 0.5f) * 2.0f * kPI;
-    const float cp = cosf(phi);
-    const float3 d = f3(cp * cosf(theta), cp * sinf(theta), sinf(phi));
+    const float2 th = sincos_nl(theta), ph = sincos_nl(phi);
+    const float cp = ph.y;
+    const float3 d = f3(cp * th.y, cp * th.x, ph.x);
     pdf = cp > 1e-7f ? env_texel_weight(s, row, col) * (float)s.env_w * (float)s.env_h / (2.0f * kPI * kPI * cp)
                      : 0.0f;
     Le = env_texel(s, row * s.env_w + col);
