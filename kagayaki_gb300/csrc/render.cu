@@ -118,6 +118,8 @@ enum Stat { kRaysC = 0, kRaysS = 1, kOverflow = 2, kNodes = 3, kTris = 4, kRaysT
 constexpr int kTailPaths = 1 << 17;
 // Idle lanes of a tail warp that take new paths together.
 constexpr int kTailRefill = 8;
+// k_compat: the largest scene it renders and its threads per block.
+constexpr int kCompatTris = 1024, kCompatThreads = 512;
 // Deferred shadow rays of the tail (unbiased estimator without the cache):
 // the first kDeferBounces bounces of a tail path leave their face-light and
 // environment shadow rays in fixed slots (path, bounce, kind) instead of
@@ -1205,6 +1207,104 @@ __global__ void __launch_bounds__(128) k_tail(Params P, int cnt_idx, int dense_n
     warp_add_u64(&P.stats[kOverflow], overflow);
 }
 
+// The reference's estimator on a small scene with a path per thread, a block
+// in step: all of its live paths' closest hits, then their shading, then their
+// shadow rays, with a barrier after each.  Its code (140 KB inlined) is larger
+// than the instruction cache: warps that drift apart each fetch all of it (66 %
+// hits, 4.8 stall cycles per instruction), in step they fetch it once.
+struct CompatCount {
+    unsigned rays_c = 0, rays_s = 0;
+    TravStats st{0, 0, 0};
+};
+
+// Runs the block's paths (live: this thread has one) to their ends, at most
+// `bounces` bounces.  All threads of the block must call it.
+__device__ __forceinline__ void compat_paths(const Params &P, PathState &ps, bool live, int bounces, CompatCount &c) {
+    const DevScene &s = P.sc;
+    for (int k = 0; k < bounces; ++k) {
+        float4 h = make_float4(kBigT, 0.0f, 0.0f, __int_as_float(-1));
+        if (live) {
+            const RayPre r = make_ray(ps.o, ps.d);
+            float bt = kBigT, u = 0.0f, v = 0.0f;
+            int bid = 0x7fffffff;
+            const int slot = trace_closest<false>(s.nodes, (unsigned)s.n_nodes, s.tri_rec, (unsigned)s.n_tris, r, bt,
+                                                  bid, u, v, c.st);
+            if (slot >= 0) h = make_float4(bt, u, v, __int_as_float(bid));
+            ++c.rays_c;
+        }
+        __syncthreads();
+        ShadeOut so{};
+        if (live) shade_compat_core(P, ps, h, so);
+        __syncthreads();
+        if (so.f_pred) {  // the reference's test: the closest hit is the light
+            const RayPre rs = make_ray(so.f_org, so.f_dir);
+            float lt = so.f_tmax, lu, lv;
+            int lid = 0x7fffffff;
+            const int ls = trace_closest<false>(s.nodes, (unsigned)s.n_nodes, s.tri_rec, (unsigned)s.n_tris, rs, lt,
+                                                lid, lu, lv, c.st);
+            if (ls >= 0 && lid == so.f_light) ps.rad = ps.rad + so.f_c;
+            ++c.rays_s;
+        }
+        if (so.e_pred) {
+            const RayPre rs = make_ray(so.spos, so.e_dir);
+            if (!trace_any<false>(s.nodes, (unsigned)s.n_nodes, s.tri_rec, (unsigned)s.n_tris, rs, kBigT, c.st))
+                ps.rad = ps.rad + so.e_c;
+            ++c.rays_s;
+        }
+        live = so.cont;
+        if (!__syncthreads_or(live)) break;
+    }
+}
+
+__device__ __forceinline__ void compat_flush(const Params &P, const CompatCount &c) {
+    warp_add_u64(&P.stats[kRaysC], c.rays_c);
+    warp_add_u64(&P.stats[kRaysS], c.rays_s);
+    warp_add_u64(&P.stats[kRaysT], c.rays_c);
+    warp_add_u64(&P.stats[kOverflow], c.st.overflow);
+}
+
+// A pixel per thread (slots in 8 x 4 tiles), the block going through the
+// call's samples one after another.  The seed chain orders a pixel's own
+// samples only (render.cuh:19,29,42), so no block waits for another's longest
+// path and a sample needs no launches.  Cornell box, 256 x 256, 16 samples:
+// 3.36 -> 2.44 ms (a wave of three launches per sample before; the same with
+// a barrier per phase 2.81; a warp going through its 32 pixels' samples alone
+// 3.30).
+__global__ void __launch_bounds__(kCompatThreads) k_compat(Params P, int spp, int bounces, float4 *frame, double *acc_sum,
+                                                double *acc_sq, int accumulate) {
+    CompatCount c;
+    for (int base = blockIdx.x * blockDim.x; base < P.npx; base += gridDim.x * blockDim.x) {
+        const int slot = base + threadIdx.x;
+        const bool mine = slot < P.npx;
+        const int px = mine ? tiled_path(P, slot) : 0;
+        float3 f = f3(0.0f, 0.0f, 0.0f);
+#pragma unroll 1
+        for (int smp = 0; smp < spp; ++smp) {
+            PathState ps;
+            ps.id = px;
+            if (mine) primary_ray(P, px, ps.d, ps.rs);
+            ps.o = f3(P.cam.CamOrg.x, P.cam.CamOrg.y, P.cam.CamOrg.z);
+            ps.T = f3(1.0f, 1.0f, 1.0f);
+            ps.rad = f3(kSINF, kSINF, kSINF);  // RayTrace.cuh:14
+            ps.pdf = 0.0f;
+            ps.depth = 0;
+            compat_paths(P, ps, mine, bounces, c);
+            f.x += ps.rad.x;
+            f.y += ps.rad.y;
+            f.z += ps.rad.z;
+            if (accumulate && mine) {
+                const float r[3] = {ps.rad.x, ps.rad.y, ps.rad.z};
+                for (int a = 0; a < 3; ++a) {
+                    acc_sum[3 * px + a] += r[a];
+                    acc_sq[3 * px + a] += (double)r[a] * r[a];
+                }
+            }
+        }
+        if (mine) frame[px] = make_float4(f.x, f.y, f.z, 0.0f);
+    }
+    compat_flush(P, c);
+}
+
 // Paths still live when the bounce limit ends the wavefront: their radiance
 // so far is final.
 __global__ void k_flush(Params P, int cnt_idx) {
@@ -1688,7 +1788,27 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
         ev_stage.push_back(-1);
         return KGK_OK;
     };
-    for (int done = 0, wave = 0; done < cfg->spp; done += spw, ++wave) {
+    // The reference's estimator on a small scene and image: a pixel per thread,
+    // all samples in one launch (k_compat).  The block goes at the pace of its
+    // longest traversal, so only while the tree is a few nodes: measured
+    // against the wave per sample, 256 x 256 pixels, 4 samples, 0.60 : 0.82 ms
+    // at 36 triangles (0.80 : 1.77 with Disney boxes), 1.05 : 0.98 at 2,562,
+    // 1.25 : 1.16 at 5,122, 2.8 : 2.0 at 1.3M.  Two rounds of one block per SM
+    // at most: 400 x 400 1.14 : 1.43 ms, 640 x 480 1.98 : 1.71.
+    const bool by_pixel = cfg->estimator == KGK_ESTIMATOR_COMPAT && s->dev.n_tris <= kCompatTris &&
+                          npx <= 2 * kCompatThreads * R.sms;
+    if (by_pixel) {
+        P.spp_wave = 1;
+        // one block per SM, whose warps are then all in step
+        const int per = std::min(kCompatThreads, std::max(32, ((npx + R.sms - 1) / R.sms + 31) & ~31));
+        KGK_TRY(stage_begin(3));
+        k_compat<<<(npx + per - 1) / per, per, 0, st>>>(P, cfg->spp, max_bounces, R.frame, R.acc_sum, R.acc_sq,
+                                                        cfg->accumulate);
+        KGK_TRY(stage_end());
+        KGK_CUDA(cudaGetLastError());
+        ++launches;
+    }
+    for (int done = by_pixel ? cfg->spp : 0, wave = 0; done < cfg->spp; done += spw, ++wave) {
         P.spp_wave = std::min(spw, cfg->spp - done);
         P.sample_base = done;
         const int n = npx * P.spp_wave;
