@@ -55,41 +55,55 @@ __device__ __forceinline__ void sb_init(kgk_svgf_buffer &b) {
     b.willApplyTemporalAccumulation = false;
 }
 
-__device__ __forceinline__ float depth_w(float d, float nd, int dx, int dy, float gx, float gy) {
-    const float top = -1.0f * fabsf(d - nd);
-    const float bottom = 1.0f * fabsf((float)dx * gx + (float)dy * gy) + kS;
-    return expf(top / bottom);
+__device__ __forceinline__ float ex2a(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float lg2a(float x) {
+    float y;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+constexpr float kLog2e = 1.44269504088896341f;
+
+// The compat weights (SVGF.cuh:187-215, 415-440).  The depth weight
+// exp(-|d - nd| / (|dx gx + dy gy| + sINF)) and the luminance weight
+// exp(-|l - nl| / (4 sd + sINF)) share one base-2 exponential of the sum of
+// their arguments, each a product with a reciprocal (the luminance one taken
+// once per pixel): an argument x carries a relative 2^-22 and so does the
+// exponential, below the 128 u of the normal weight's seven squarings.
+__device__ __forceinline__ float depth_arg(float d, float nd, float slope) {
+    return __fdividef(-kLog2e * fabsf(d - nd), fabsf(slope) + kS);
 }
 __device__ __forceinline__ float normal_w(float3 n, float3 m) {
     float c = fmaxf(0.0f, dot3(n, m));
     c *= c; c *= c; c *= c; c *= c; c *= c; c *= c; c *= c;  // ^128
     return c;
 }
-__device__ __forceinline__ float lum_w(float l, float nl, float sd) {
-    const float top = -1.0f * fabsf(l - nl);
-    const float bottom = 4.0f * sd + kS;
-    return expf(top / bottom);
-}
 
 struct CompatArgs {
     int W, H, frame;
     kgk_vec *R, *F;
     kgk_svgf_buffer *P, *C;
-    float *M1, *M2, *sd, *gz, *s1, *s2, *sw, *var;
+    float *M1, *M2, *sd, *gz, *s1, *s2, *sw;
     unsigned char *spatial;
     kgk_vec *R2;
-    // the a-trous passes' per-pixel guide, packed from the records once their
-    // fields are final (k_c_gauss2): normal and depth, ObjectID and MaterialID
+    // The spatial passes' per-pixel guide, packed from the records: normal and
+    // depth.
     float4 *gnd;
-    int2 *gom;
-    // the center pixel's albedo and willApplyATrousFilter (w = 1 or 0),
-    // final from k_c_gauss2 on: a pass reads 16 B instead of two sectors of
-    // the 112-byte record
+    // MaterialID and variance, the variance's sign bit set where ObjectID is -1
+    // (variances are never negative).  Before k_c_var4: ObjectID, MaterialID.
+    int2 *mv, *mv2;
+    // the center pixel's albedo and willApplyATrousFilter (w = 1 or 0)
     float4 *galf;
     // each pass's input radiance divided by (albedo + sINF), with its
     // luminance in w: written by the pass before (ping-pong), so a tap reads
     // it instead of dividing
     float4 *dm, *dm2;
+    // ColorHistory of the records while the passes run (over M1, M2, s1 and
+    // s2, whose last reader is k_c_var4)
+    kgk_vec *hist;
 };
 
 #define FOR_PIXELS(n) for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < (n); p += gridDim.x * blockDim.x)
@@ -129,61 +143,87 @@ ToneTable tone_table() {
     return T;
 }
 
-__global__ void k_c_prologue(CompatArgs a) {
-    FOR_PIXELS(a.W * a.H) {
-        float3 r = v3(a.R[p]);
-        if (!isfinite(len3(r))) a.R[p] = kv(f3(0.0f, 0.0f, 0.0f));
-        if (a.frame == 0) sb_init(a.P[p]);
-        if (a.P[p].MomentOne == -1.0f) {
-            const float m1 = lumf(div3(v3(a.R[p]), v3(a.C[p].Albedo)));
-            a.C[p].MomentOne = m1;
-            a.C[p].MomentTwo = m1 * m1;
-        }
-        a.F[p] = kv(f3(0.0f, 0.0f, 0.0f));
-    }
+// frame 0: every previous record initialised (SVGF.cuh:502-504), stored as
+// consecutive words: T = uint4, or unsigned where the caller's array does not
+// start on 16 bytes.
+constexpr int kRecWords = (int)(sizeof(kgk_svgf_buffer) / 4);
+template <class T>
+__global__ void __launch_bounds__(256) k_c_init_prev(kgk_svgf_buffer *P, size_t npx) {
+    __shared__ __align__(16) unsigned s_rec[kRecWords];
+    if (threadIdx.x < kRecWords) s_rec[threadIdx.x] = 0u;  // the padding too
+    __syncthreads();
+    if (threadIdx.x == 0) sb_init(*reinterpret_cast<kgk_svgf_buffer *>(s_rec));
+    __syncthreads();
+    constexpr unsigned kPer = sizeof(kgk_svgf_buffer) / sizeof(T);
+    const T *src = reinterpret_cast<const T *>(s_rec);
+    T *dst = reinterpret_cast<T *>(P);
+    const size_t n = npx * kPer;
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256)
+        dst[i] = src[i % kPer];
 }
 
-// TemporalAccumulation (SVGF.cuh:50-98)
-__global__ void k_c_temporal(CompatArgs a) {
-    const int W = a.W, H = a.H;
-    FOR_PIXELS(W * H) {
-        const kgk_svgf_buffer &c = a.C[p];
-        if (len3(v3(c.Emission)) != 0.0f) continue;
-        const int px = c.PosLastFrameI[0], py = c.PosLastFrameI[1];
-        const float s = c.PosLastFrameF[0] - (float)px, t = c.PosLastFrameF[1] - (float)py;
-        const int ox[4] = {0, 1, 0, 1}, oy[4] = {0, 0, 1, 1};
-        const float w[4] = {(1 - s) * (1 - t), s * (1 - t), (1 - s) * t, s * t};
-        float3 sum = f3(0.0f, 0.0f, 0.0f);
-        float swt = 0.0f;
-        for (int i = 0; i < 4; ++i) {
-            const int qx = px + ox[i], qy = py + oy[i];
-            if (qx < 0 || qx >= W || qy < 0 || qy >= H) continue;
-            const kgk_svgf_buffer &q = a.P[W * qy + qx];
-            if (q.MaterialID == c.MaterialID && q.willApplyTemporalAccumulation) {
-                sum += v3(q.ColorHistory) * w[i];
-                swt += w[i];
-            }
-        }
-        if (swt == 0.0f) continue;
-        const float3 hist = sum / swt;
-        a.R[p] = kv(v3(a.R[p]) * 0.2f + hist * 0.8f);
-    }
-}
-
-// VarianceEstimation, before the first barrier (SVGF.cuh:114-145)
-__global__ void k_c_var1(CompatArgs a) {
+// Everything up to VarianceEstimation's spatial filter that a pixel does by
+// itself: the radiance made finite (SVGF.cuh:498-500), TemporalAccumulation
+// (SVGF.cuh:50-98), the moments and the choice between their temporal update
+// and the spatial estimate (SVGF.cuh:114-165).  The records' moments of
+// SVGF.cuh:506-512 are not stored: every pixel's are replaced here or in
+// k_c_var4 before they are read.  At frame 0 the previous records hold no
+// history and no samples, so they are not read.
+__global__ void k_c_front(CompatArgs a) {
     const int W = a.W, H = a.H;
     FOR_PIXELS(W * H) {
         const int x = p % W, y = p / W;
-        const kgk_svgf_buffer &c = a.C[p];
-        const float l = lumf(div3(v3(a.R[p]), v3(c.Albedo) + f3(kS, kS, kS)));
-        a.M1[p] = l;
-        a.M2[p] = l * l;
-        bool sp = c.PosLastFrameI[0] == -1;
-        if (!sp) {
-            const int prev = W * c.PosLastFrameI[1] + c.PosLastFrameI[0];
-            sp = (prev < 0 || prev >= W * H) ? true : a.P[prev].sampleNum < 3;
+        kgk_svgf_buffer &c = a.C[p];
+        const kgk_vec r0 = a.R[p];
+        float3 r = v3(r0);
+        bool store = false;
+        if (!isfinite(len3(r))) {
+            r = f3(0.0f, 0.0f, 0.0f);
+            store = true;
         }
+        const int px = c.PosLastFrameI[0], py = c.PosLastFrameI[1], mat = c.MaterialID;
+        if (a.frame != 0 && len3(v3(c.Emission)) == 0.0f) {
+            const float s = c.PosLastFrameF[0] - (float)px, t = c.PosLastFrameF[1] - (float)py;
+            const int ox[4] = {0, 1, 0, 1}, oy[4] = {0, 0, 1, 1};
+            const float w[4] = {(1 - s) * (1 - t), s * (1 - t), (1 - s) * t, s * t};
+            float3 sum = f3(0.0f, 0.0f, 0.0f);
+            float swt = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int qx = px + ox[i], qy = py + oy[i];
+                if (qx < 0 || qx >= W || qy < 0 || qy >= H) continue;
+                const kgk_svgf_buffer &q = a.P[W * qy + qx];
+                if (q.MaterialID == mat && q.willApplyTemporalAccumulation) {
+                    sum += v3(q.ColorHistory) * w[i];
+                    swt += w[i];
+                }
+            }
+            if (swt != 0.0f) {
+                r = r * 0.2f + (sum / swt) * 0.8f;
+                store = true;
+            }
+        }
+        if (store) a.R[p] = kv(r);
+        const float l = lumf(div3(r, v3(c.Albedo) + f3(kS, kS, kS)));
+        float m1 = l, m2 = l * l;
+        bool sp = a.frame == 0 || px == -1;
+        if (!sp) {
+            const int prev = W * py + px;
+            if (prev < 0 || prev >= W * H || a.P[prev].sampleNum < 3) {
+                sp = true;
+            } else {
+                const int n = a.P[prev].sampleNum + 1;
+                float cw = 1.0f / 5.0f;
+                if (n < 5) cw = 1.0f / (float)n;
+                m1 = (1.0f - cw) * a.P[prev].MomentOne + cw * m1;
+                m2 = (1.0f - cw) * a.P[prev].MomentTwo + cw * m2;
+                c.sampleNum = n;
+                c.MomentOne = m1;
+                c.MomentTwo = m2;
+            }
+        }
+        a.M1[p] = m1;
+        a.M2[p] = m2;
         a.spatial[p] = sp ? 1 : 0;
         const int dx = x < W / 2 ? 1 : -1, dy = y < H / 2 ? 1 : -1;
         const float d = c.Depth;
@@ -191,23 +231,7 @@ __global__ void k_c_var1(CompatArgs a) {
         a.gz[2 * p + 1] = (a.C[W * (y + dy) + x].Depth - d) / (float)dy;
         // the guide k_c_var3 reads (the records as they are before k_c_var4)
         a.gnd[p] = make_float4(c.Normal.x, c.Normal.y, c.Normal.z, d);
-        a.gom[p] = make_int2(c.ObjectID, c.MaterialID);
-    }
-}
-
-__global__ void k_c_var2(CompatArgs a) {
-    const int W = a.W;
-    FOR_PIXELS(W * a.H) {
-        if (a.spatial[p]) continue;
-        kgk_svgf_buffer &c = a.C[p];
-        const int prev = W * c.PosLastFrameI[1] + c.PosLastFrameI[0];
-        c.sampleNum = a.P[prev].sampleNum + 1;
-        float cw = 1.0f / 5.0f;
-        if (c.sampleNum < 5) cw = 1.0f / (float)c.sampleNum;
-        c.MomentOne = (1.0f - cw) * a.P[prev].MomentOne + cw * a.M1[p];
-        c.MomentTwo = (1.0f - cw) * a.P[prev].MomentTwo + cw * a.M2[p];
-        a.M1[p] = c.MomentOne;
-        a.M2[p] = c.MomentTwo;
+        a.mv[p] = make_int2(c.ObjectID, mat);
     }
 }
 
@@ -235,7 +259,7 @@ __global__ void __launch_bounds__(256) k_c_var3(CompatArgs a) {
         if (gx < 0 || gx >= W || gy < 0 || gy >= H) continue;
         const int q = W * gy + gx;
         s_nd[i] = a.gnd[q];
-        s_om[i] = a.gom[q];
+        s_om[i] = a.mv[q];
         s_m[i] = make_float2(a.M1[q], a.M2[q]);
     }
     __syncthreads();
@@ -268,7 +292,7 @@ __global__ void __launch_bounds__(256) k_c_var3(CompatArgs a) {
             if (om.x == -1) continue;
             const float4 qn = s_nd[t];
             const float wm = cmat == om.y ? 1.0f : 0.0f;
-            const float wz = depth_w(cn.w, qn.w, kx, ky, gzx, gzy);
+            const float wz = ex2a(depth_arg(cn.w, qn.w, (float)kx * gzx + (float)ky * gzy));
             const float wn = normal_w(n, f3(qn));
             const float w = hx * hy * wz * wn * wm;
             s1 += w * s_m[t].x;
@@ -281,104 +305,116 @@ __global__ void __launch_bounds__(256) k_c_var3(CompatArgs a) {
     a.sw[p] = sw;
 }
 
+// The rest of VarianceEstimation (SVGF.cuh:226-275): records without an object
+// or an estimate are reset, the others get their moments; the variance goes to
+// mv (the records take their final one in k_c_final).
 __global__ void k_c_var4(CompatArgs a) {
     const int W = a.W;
     FOR_PIXELS(W * a.H) {
         kgk_svgf_buffer &c = a.C[p];
-        if (c.ObjectID == -1 || (a.spatial[p] && a.sw[p] == 0.0f)) {
+        const int2 om = a.mv[p];
+        const bool sp = a.spatial[p];
+        const float sw = a.sw[p];
+        if (om.x == -1 || (sp && sw == 0.0f)) {
             a.F[p] = a.R[p];
             sb_init(c);
             c.willApplyATrousFilter = false;
-        } else if (a.spatial[p]) {
-            c.MomentOne = a.s1[p] / a.sw[p];
-            c.MomentTwo = a.s2[p] / a.sw[p];
-            if (c.PosLastFrameI[0] == -1) c.sampleNum = 1;
-            else c.sampleNum = a.P[W * c.PosLastFrameI[1] + c.PosLastFrameI[0]].sampleNum + 1;
+            a.gnd[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            a.mv[p] = make_int2(-1, (int)0x80000000);
+            continue;
         }
+        float m1, m2;
+        if (sp) {
+            m1 = a.s1[p] / sw;
+            m2 = a.s2[p] / sw;
+            c.MomentOne = m1;
+            c.MomentTwo = m2;
+            if (a.frame == 0 || c.PosLastFrameI[0] == -1) c.sampleNum = 1;
+            else c.sampleNum = a.P[W * c.PosLastFrameI[1] + c.PosLastFrameI[0]].sampleNum + 1;
+        } else {
+            m1 = a.M1[p];
+            m2 = a.M2[p];
+        }
+        a.mv[p] = make_int2(om.y, __float_as_int(fminf(fmaxf(0.0f, m2 - m1 * m1), 1000.0f)));
     }
 }
 
-__global__ void k_c_var5(CompatArgs a) {
-    FOR_PIXELS(a.W * a.H) {
-        kgk_svgf_buffer &c = a.C[p];
-        if (c.ObjectID == -1) continue;
-        c.Variance = fmaxf(0.0f, c.MomentTwo - c.MomentOne * c.MomentOne);
-        if (c.Variance > 1000) c.Variance = 1000;
-    }
-}
-
-// ApplyGaussianFilterToVar (SVGF.cuh:277-344)
-__global__ void k_c_gauss1(CompatArgs a) {
+// ApplyGaussianFilterToVar (SVGF.cuh:277-344), and what the a-trous passes
+// read: the records' fields are final from here to their end.
+__global__ void k_c_gauss(CompatArgs a) {
     const int W = a.W, H = a.H;
     FOR_PIXELS(W * H) {
         const int x = p % W, y = p / W;
         float sv = 0, sw = 0;
+#pragma unroll
         for (int kx = -1; kx <= 1; ++kx) {
             const float hx = cKG[kx + 1];
             const int nx = x + kx;
             if (nx < 0 || nx >= W) continue;
+#pragma unroll
             for (int ky = -1; ky <= 1; ++ky) {
-                const float hy = cKG[ky + 1];
                 const int ny = y + ky;
                 if (ny < 0 || ny >= H) continue;
-                const kgk_svgf_buffer &d = a.C[W * ny + nx];
-                if (d.ObjectID == -1) continue;
-                const float w = hx * hy;
-                sv += w * d.Variance;
+                const int v = a.mv[W * ny + nx].y;
+                if (v < 0) continue;
+                const float w = hx * cKG[ky + 1];
+                sv += w * __int_as_float(v);
                 sw += w;
             }
         }
-        a.s1[p] = sv;
-        a.sw[p] = sw;
-    }
-}
-
-__global__ void k_c_gauss2(CompatArgs a) {
-    FOR_PIXELS(a.W * a.H) {
         kgk_svgf_buffer &c = a.C[p];
-        a.sd[p] = 0.0f;
-        if (a.s1[p] == 0.0f && a.sw[p] != 0.0f) {
-            a.F[p] = a.R[p];
-            c.willApplyATrousFilter = false;
-        } else if (a.sw[p] == 0.0f) {
+        const int2 own = a.mv[p];
+        float var = __int_as_float(own.y & 0x7fffffff), sd = 0.0f;
+        bool filt = c.willApplyATrousFilter;
+        if (sw == 0.0f) {
             c.MomentOne = -1.0f;
             c.MomentTwo = -1.0f;
             c.sampleNum = 0;
+        }
+        if (sv == 0.0f || sw == 0.0f) {
+            filt = false;
             c.willApplyATrousFilter = false;
         } else {
-            c.Variance = a.s1[p] / a.sw[p];
-            a.sd[p] = sqrtf(a.s1[p] / a.sw[p]);
+            var = sv / sw;
+            sd = sqrtf(var);
         }
-        a.var[p] = c.Variance;
-        // the records' normal, depth, ids and albedo are final from here to
-        // the end of the a-trous passes, and so is R before the first pass
-        a.gnd[p] = make_float4(c.Normal.x, c.Normal.y, c.Normal.z, c.Depth);
-        a.gom[p] = make_int2(c.ObjectID, c.MaterialID);
-        a.galf[p] = make_float4(c.Albedo.x, c.Albedo.y, c.Albedo.z, c.willApplyATrousFilter ? 1.0f : 0.0f);
-        const float3 dc = div3(v3(a.R[p]), v3(c.Albedo) + f3(kS, kS, kS));
+        a.sd[p] = sd;
+        a.mv2[p] = make_int2(own.x, __float_as_int(var) | (own.y & (int)0x80000000));
+        const float3 alb = v3(c.Albedo);
+        a.galf[p] = make_float4(alb.x, alb.y, alb.z, filt ? 1.0f : 0.0f);
+        const float3 dc = div3(v3(a.R[p]), alb + f3(kS, kS, kS));
         a.dm[p] = make_float4(dc.x, dc.y, dc.z, lumf(dc));
+        a.hist[p] = c.ColorHistory;
         // the a-trous passes' depth gradient (SVGF.cuh:366-372), from the
-        // records as k_c_var4 left them; k_c_var3 was the last reader of gz
-        const int W = a.W, x = p % W, y = p / W;
-        const int dx = x < W / 2 ? 1 : -1, dy = y < a.H / 2 ? 1 : -1;
-        a.gz[2 * p] = (a.C[W * y + x + dx].Depth - c.Depth) / (float)dx;
-        a.gz[2 * p + 1] = (a.C[W * (y + dy) + x].Depth - c.Depth) / (float)dy;
+        // records as k_c_var4 left them
+        const int dx = x < W / 2 ? 1 : -1, dy = y < H / 2 ? 1 : -1;
+        const float d = a.gnd[p].w;
+        a.gz[2 * p] = (a.gnd[W * y + x + dx].w - d) / (float)dx;
+        a.gz[2 * p + 1] = (a.gnd[W * (y + dy) + x].w - d) / (float)dy;
     }
 }
 
 // One a-trous stage (SVGF.cuh:347-474) of pixel p = (x, y) at step 2^stage.
 // Reads go through Src: the global arrays (k_c_atrous) or a shared-memory
-// tile of them (k_c_atrous_tile); either way every tap is the reference's
-// expression in its order, so both give the same bits.  A tap's neighbour
-// radiance comes demodulated with its luminance (dm, written by the pass
-// before) instead of being divided by its albedo at every tap.
+// tile of them (k_c_atrous_tile); every tap is the same expression in the
+// reference's order.  A tap's neighbour radiance comes demodulated with its
+// luminance (dm, written by the pass before) instead of being divided by its
+// albedo at every tap.  The filtered image and the records' flags and history
+// take their last pass's values, so they are stored once, in k_c_final.
+// Instruction issue bounds a pass (two IEEE divisions and two expf a tap
+// before, one reciprocal and one ex2 now), then shared memory (40 B a tap).
+// 1080p: a pass 202 / 195 / 201 / 247 / 244 us at steps 1 / 2 / 4 / 8 / 16 ->
+// 98 / 99 / 118 / 144 / 146; the call 6.35 -> 4.15 ms, with the front and
+// variance kernels' passes over the 112-byte records 1.19 -> 0.65 ms.  Error
+// against 64 bits over 64 x 64 to 2560 x 1440, with and without motion:
+// 3.6e-7 to 5.4e-7 before and after.
 struct CompatIO {
     const kgk_vec *Rin;
     kgk_vec *Rout;
     const float4 *dmin;
     float4 *dmout;
-    const float *vin;
-    float *vout;
+    const int2 *vin;
+    int2 *vout;
 };
 
 template <class Src>
@@ -387,55 +423,49 @@ __device__ __forceinline__ void compat_atrous_px(const CompatArgs &a, const Comp
     const int W = a.W, H = a.H, p = W * y + x, step = 1 << stage;
     const float4 af = a.galf[p];
     const float4 g = S.nd(0, 0);
-    const int2 om = S.om(0, 0);
+    const int2 om = S.mv(0, 0);
     const float4 dcl = S.dm(0, 0);
-    const float3 dc = f3(dcl);
-    const float l = dcl.w;
-    const float d = g.w;
+    const float l = dcl.w, d = g.w;
     const float gx = a.gz[2 * p], gy = a.gz[2 * p + 1];
     const float3 n = f3(g);
-    const float sdv = a.sd[p];
     const bool filt = af.w != 0.0f;
+    // the luminance weight's factor of |l - nl| (0: no luminance weight)
+    const float rl = filt ? __fdividef(-kLog2e, 4.0f * a.sd[p] + kS) : 0.0f;
+    // a tap brighter than this is left out (SVGF.cuh:405-411, whose first two
+    // bounds compare in double)
+    const float bright = (double)l > 0.5 ? 5 * l : (double)l > 0.1 ? 50 * l : l > kS ? 100 * l : INFINITY;
+    const float cvar = __int_as_float(om.y & 0x7fffffff);
     float3 srad = f3(0.0f, 0.0f, 0.0f);
     float svar = 0.0f, swt = 0.0f;
 #pragma unroll
     for (int ki = 0; ki < 25; ++ki) {
         const float h = cKW[ki];
         const int ox = (ki % 5 - 2) * step, oy = (ki / 5 - 2) * step;
-        const int qx = x + ox, qy = y + oy;
-        if (qx < 0 || qx >= W || qy < 0 || qy >= H) continue;
         if (ki == 12) {
-            svar += h * h * S.v(0, 0);
-            srad += dc * h;
+            svar += h * h * cvar;
+            srad += f3(dcl) * h;
             swt += h;
             continue;
         }
-        const int2 eo = S.om(ox, oy);
-        if (eo.x == -1) continue;
+        const int qx = x + ox, qy = y + oy;
+        if (qx < 0 || qx >= W || qy < 0 || qy >= H) continue;
+        const int2 eo = S.mv(ox, oy);
         const float4 em = S.dm(ox, oy);
-        const float3 nr = f3(em);
-        const float nl = em.w;
-        if (((double)l > 0.5 && nl > 5 * l) || ((double)l > 0.1 && nl > 50 * l) || (l > kS && nl > 100 * l))
-            continue;
+        if (eo.y < 0 || em.w > bright) continue;
         const float4 eg = S.nd(ox, oy);
-        const float wm = om.y == eo.y ? 1.0f : 0.0f;
-        const float wz = depth_w(d, eg.w, qx, qy, gx, gy);  // absolute coordinates, SVGF.cuh:426
-        const float wn = normal_w(n, f3(eg));
-        const float wl = lum_w(l, nl, sdv);
-        const float w = filt ? h * wz * wn * wl * wm : h * wz * wn * wm;
-        srad += nr * w;
-        svar += w * w * S.v(ox, oy);
+        // absolute coordinates in the depth weight, SVGF.cuh:426
+        const float e = depth_arg(d, eg.w, (float)qx * gx + (float)qy * gy) + fminf(fabsf(l - em.w), 3e38f) * rl;
+        float w = h * ex2a(e) * normal_w(n, f3(eg));
+        w = om.x == eo.x ? w : 0.0f;
+        srad += f3(em) * w;
+        svar += w * w * __int_as_float(eo.y);
         swt += w;
     }
     const kgk_vec rin = io.Rin[p];
-    const float vc = S.v(0, 0);
-    if (om.x == -1 || swt < 1e-6f || swt * swt < 1e-6f) {
+    if (om.y < 0 || swt < 1e-6f || swt * swt < 1e-6f) {
         io.Rout[p] = rin;
-        io.vout[p] = vc;
+        io.vout[p] = om;
         io.dmout[p] = dcl;
-        if (om.x == -1) return;
-        a.F[p] = rin;
-        a.C[p].willApplyTemporalAccumulation = true;
         return;
     }
     const float3 alb = f3(af);
@@ -443,33 +473,27 @@ __device__ __forceinline__ void compat_atrous_px(const CompatArgs &a, const Comp
     const float fv = svar / (swt * swt);
     const float cw = 0.2f;
     const float3 o = (fl * alb) * cw + v3(rin) * (1 - cw);
-    a.F[p] = kv(o);
     io.Rout[p] = kv(o);
     const float3 od = div3(o, alb + f3(kS, kS, kS));
     io.dmout[p] = make_float4(od.x, od.y, od.z, lumf(od));
-    io.vout[p] = filt ? cw * vc + (1 - cw) * fv : vc;
-    if (stage == 0) {
-        a.C[p].ColorHistory = kv(o);
-        a.C[p].willApplyTemporalAccumulation = true;
-    }
+    io.vout[p] = make_int2(om.x, __float_as_int(filt ? cw * cvar + (1 - cw) * fv : cvar));
+    if (stage == 0) a.hist[p] = kv(o);
 }
 
 // Taps read straight from the global arrays (offsets from pixel p).
 struct CompatGlobal {
     const float4 *gnd_, *dm_;
-    const int2 *gom_;
-    const float *v_;
+    const int2 *mv_;
     int p, W;
     __device__ float4 nd(int ox, int oy) const { return gnd_[p + W * oy + ox]; }
-    __device__ int2 om(int ox, int oy) const { return gom_[p + W * oy + ox]; }
+    __device__ int2 mv(int ox, int oy) const { return mv_[p + W * oy + ox]; }
     __device__ float4 dm(int ox, int oy) const { return dm_[p + W * oy + ox]; }
-    __device__ float v(int ox, int oy) const { return v_[p + W * oy + ox]; }
 };
 
 __global__ void k_c_atrous(CompatArgs a, CompatIO io, int stage) {
     const int W = a.W;
     FOR_PIXELS(W * a.H) {
-        const CompatGlobal S{a.gnd, io.dmin, a.gom, io.vin, p, W};
+        const CompatGlobal S{a.gnd, io.dmin, io.vin, p, W};
         compat_atrous_px(a, io, S, p % W, p / W, stage);
     }
 }
@@ -481,19 +505,17 @@ __global__ void k_c_atrous(CompatArgs a, CompatIO io, int stage) {
 // tap's bounds test comes first).
 template <int kStep> struct CTile {
     static constexpr int R = 2 * kStep, SX = kCTX + 2 * R, SY = kCTY + 2 * R, N = SX * SY;
-    static constexpr size_t kSmem = (size_t)N * (2 * sizeof(float4) + sizeof(int2) + sizeof(float));
+    static constexpr size_t kSmem = (size_t)N * (2 * sizeof(float4) + sizeof(int2));
 };
 
 // Taps read from a tile of row length SX (offsets from entry c).
 template <int SX> struct CompatShared {
     const float4 *snd, *sdm;
-    const int2 *som;
-    const float *sv;
+    const int2 *smv;
     int c;
     __device__ float4 nd(int ox, int oy) const { return snd[c + SX * oy + ox]; }
-    __device__ int2 om(int ox, int oy) const { return som[c + SX * oy + ox]; }
+    __device__ int2 mv(int ox, int oy) const { return smv[c + SX * oy + ox]; }
     __device__ float4 dm(int ox, int oy) const { return sdm[c + SX * oy + ox]; }
-    __device__ float v(int ox, int oy) const { return sv[c + SX * oy + ox]; }
 };
 
 template <int kStep>
@@ -502,8 +524,7 @@ __global__ void __launch_bounds__(256) k_c_atrous_tile(CompatArgs a, CompatIO io
     extern __shared__ __align__(16) unsigned char smem[];
     float4 *s_nd = (float4 *)smem;
     float4 *s_dm = s_nd + T::N;
-    int2 *s_om = (int2 *)(s_dm + T::N);
-    float *s_v = (float *)(s_om + T::N);
+    int2 *s_mv = (int2 *)(s_dm + T::N);
     const int W = a.W, H = a.H;
     const int x0 = blockIdx.x * kCTX - T::R, y0 = blockIdx.y * kCTY - T::R;
     for (int i = threadIdx.y * kCTX + threadIdx.x; i < T::N; i += kCTX * kCTY) {
@@ -512,13 +533,12 @@ __global__ void __launch_bounds__(256) k_c_atrous_tile(CompatArgs a, CompatIO io
         const int q = W * gy + gx;
         s_nd[i] = a.gnd[q];
         s_dm[i] = io.dmin[q];
-        s_om[i] = a.gom[q];
-        s_v[i] = io.vin[q];
+        s_mv[i] = io.vin[q];
     }
     __syncthreads();
     const int x = blockIdx.x * kCTX + threadIdx.x, y = blockIdx.y * kCTY + threadIdx.y;
     if (x >= W || y >= H) return;
-    const CompatShared<T::SX> S{s_nd, s_dm, s_om, s_v, T::SX * ((int)threadIdx.y + T::R) + (int)threadIdx.x + T::R};
+    const CompatShared<T::SX> S{s_nd, s_dm, s_mv, T::SX * ((int)threadIdx.y + T::R) + (int)threadIdx.x + T::R};
     compat_atrous_px(a, io, S, x, y, kStep == 1 ? 0 : kStep == 2 ? 1 : 2);
 }
 
@@ -528,20 +548,18 @@ __global__ void __launch_bounds__(256) k_c_atrous_tile(CompatArgs a, CompatIO io
 // tap comes from shared memory and the staging reads are coalesced.
 template <int kStep> struct CRows {
     static constexpr int T = 256, R = 2 * kStep, SX = T + 2 * R, N = 5 * SX;
-    static constexpr size_t kSmem = (size_t)N * (2 * sizeof(float4) + sizeof(int2) + sizeof(float));
+    static constexpr size_t kSmem = (size_t)N * (2 * sizeof(float4) + sizeof(int2));
 };
 
 // Taps read from the five staged rows (row pitch SX, one row per step).
 template <int SX, int kStep> struct CompatRows {
     const float4 *snd, *sdm;
-    const int2 *som;
-    const float *sv;
+    const int2 *smv;
     int c;
     __device__ int at(int ox, int oy) const { return c + SX * (oy / kStep) + ox; }
     __device__ float4 nd(int ox, int oy) const { return snd[at(ox, oy)]; }
-    __device__ int2 om(int ox, int oy) const { return som[at(ox, oy)]; }
+    __device__ int2 mv(int ox, int oy) const { return smv[at(ox, oy)]; }
     __device__ float4 dm(int ox, int oy) const { return sdm[at(ox, oy)]; }
-    __device__ float v(int ox, int oy) const { return sv[at(ox, oy)]; }
 };
 
 template <int kStep>
@@ -550,8 +568,7 @@ __global__ void __launch_bounds__(256) k_c_atrous_rows(CompatArgs a, CompatIO io
     extern __shared__ __align__(16) unsigned char smem[];
     float4 *s_nd = (float4 *)smem;
     float4 *s_dm = s_nd + T::N;
-    int2 *s_om = (int2 *)(s_dm + T::N);
-    float *s_v = (float *)(s_om + T::N);
+    int2 *s_mv = (int2 *)(s_dm + T::N);
     const int W = a.W, H = a.H, y = blockIdx.y;
     const int x0 = blockIdx.x * T::T - T::R;
     for (int i = threadIdx.x; i < T::N; i += T::T) {
@@ -560,67 +577,71 @@ __global__ void __launch_bounds__(256) k_c_atrous_rows(CompatArgs a, CompatIO io
         const int q = W * gy + gx;
         s_nd[i] = a.gnd[q];
         s_dm[i] = io.dmin[q];
-        s_om[i] = a.gom[q];
-        s_v[i] = io.vin[q];
+        s_mv[i] = io.vin[q];
     }
     __syncthreads();
     const int x = blockIdx.x * T::T + threadIdx.x;
     if (x >= W) return;
     constexpr int stage = kStep == 8 ? 3 : kStep == 16 ? 4 : kStep == 32 ? 5 : 6;
     static_assert((1 << stage) == kStep, "row-tile steps are 8, 16, 32 and 64");
-    const CompatRows<T::SX, kStep> S{s_nd, s_dm, s_om, s_v, 2 * T::SX + (int)threadIdx.x + T::R};
+    const CompatRows<T::SX, kStep> S{s_nd, s_dm, s_mv, 2 * T::SX + (int)threadIdx.x + T::R};
     compat_atrous_px(a, io, S, x, y, stage);
 }
 
-__global__ void k_c_final(CompatArgs a, const float *var) {
+// The records, the result and the filtered image after the last pass (its
+// output radiance Rl): pixels without an object keep the image k_c_var4 gave
+// them.
+__global__ void k_c_final(CompatArgs a, const kgk_vec *Rl, const int2 *mv) {
     FOR_PIXELS(a.W * a.H) {
-        a.C[p].Variance = var[p];
-        a.R[p] = a.C[p].ColorHistory;
+        const int v = mv[p].y;
+        kgk_svgf_buffer &c = a.C[p];
+        const kgk_vec h = a.hist[p];
+        if (v >= 0) {
+            a.F[p] = Rl[p];
+            c.willApplyTemporalAccumulation = true;
+        }
+        c.Variance = __int_as_float(v & 0x7fffffff);
+        c.ColorHistory = h;
+        a.R[p] = h;
     }
 }
 
-__global__ void k_copy_vec(const kgk_vec *src, kgk_vec *dst, int n) {
-    FOR_PIXELS(n) dst[p] = src[p];
-}
-
-// Scratch of the compat pipeline, carved from one block: M1, M2, sd, gz (two
-// arrays), s1, s2, sw, var, var2 at `fl` bytes each, then R2 (`vec` bytes),
-// the guide (gnd, 16 B a pixel), the two demodulated radiance buffers (dm,
-// dm2, 16 B each), albedo + filter flag (galf, 16 B), the ids (gom, 8 B),
-// then the per-pixel spatial flags;
-// every array starts on a 256-byte boundary.  Returns var2, the second
-// variance buffer of the a-trous passes.
+// Scratch of the compat pipeline, carved from one block: M1, M2, s1, s2 (then
+// hist over these four), sd, gz (two arrays), sw at `fl` bytes each, then R2
+// (`vec` bytes), the guide (gnd, 16 B a pixel), the two demodulated radiance
+// buffers (dm, dm2, 16 B each), albedo + filter flag (galf, 16 B), material +
+// variance twice (mv, mv2, 8 B each), then the per-pixel spatial flags; every
+// array starts on a 256-byte boundary.
 constexpr size_t scratch_up(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr size_t compat_fl(size_t npx) { return scratch_up(npx * sizeof(float)); }
 constexpr size_t compat_vec(size_t npx) { return scratch_up(npx * sizeof(kgk_vec)); }
 constexpr size_t compat_scratch_bytes(size_t npx) {
-    return 10 * compat_fl(npx) + 5 * compat_vec(npx) + scratch_up(npx * sizeof(int2)) + npx;
+    return 8 * compat_fl(npx) + 5 * compat_vec(npx) + 2 * scratch_up(npx * sizeof(int2)) + npx;
 }
 
-float *carve_compat(CompatArgs &a, unsigned char *b, size_t fl, size_t vec) {
+void carve_compat(CompatArgs &a, unsigned char *b, size_t fl, size_t vec) {
+    a.hist = (kgk_vec *)b;  // 4 fl >= vec
     a.M1 = (float *)b; b += fl;
     a.M2 = (float *)b; b += fl;
-    a.sd = (float *)b; b += fl;
-    a.gz = (float *)b; b += 2 * fl;
     a.s1 = (float *)b; b += fl;
     a.s2 = (float *)b; b += fl;
+    a.sd = (float *)b; b += fl;
+    a.gz = (float *)b; b += 2 * fl;
     a.sw = (float *)b; b += fl;
-    a.var = (float *)b; b += fl;
-    float *var2 = (float *)b; b += fl;
     a.R2 = (kgk_vec *)b; b += vec;
     a.gnd = (float4 *)b; b += vec;
     a.dm = (float4 *)b; b += vec;
     a.dm2 = (float4 *)b; b += vec;
     a.galf = (float4 *)b; b += vec;
-    a.gom = (int2 *)b; b += scratch_up(vec / 2);
+    a.mv = (int2 *)b; b += scratch_up(vec / 2);
+    a.mv2 = (int2 *)b; b += scratch_up(vec / 2);
     a.spatial = b;
-    return var2;
 }
 
 // Queues the compat pipeline (SVGF.cuh:495-522, every __syncthreads a kernel
 // boundary) on `st` and waits for it.  Every scratch word is written by an
 // earlier kernel of the same call before any kernel reads it.
-kgk_status launch_compat(CompatArgs &a, float *var2, int repeats, int stages, cudaStream_t st) {
+kgk_status launch_compat(CompatArgs &a, int repeats, int stages, cudaStream_t st) {
     const size_t npx = (size_t)a.W * a.H;
     const int g = (int)std::min<size_t>((npx + 255) / 256, 65535);
     KGK_CUDA(cudaFuncSetAttribute(k_c_atrous_tile<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -629,19 +650,18 @@ kgk_status launch_compat(CompatArgs &a, float *var2, int repeats, int stages, cu
                                   (int)CRows<8>::kSmem));
     KGK_CUDA(cudaFuncSetAttribute(k_c_atrous_rows<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)CRows<16>::kSmem));
-    k_c_prologue<<<g, 256, 0, st>>>(a);
-    k_c_temporal<<<g, 256, 0, st>>>(a);
-    k_c_var1<<<g, 256, 0, st>>>(a);
-    k_c_var2<<<g, 256, 0, st>>>(a);
+    if (a.frame == 0) {
+        if (reinterpret_cast<uintptr_t>(a.P) % 16 == 0) k_c_init_prev<uint4><<<g, 256, 0, st>>>(a.P, npx);
+        else k_c_init_prev<unsigned><<<g, 256, 0, st>>>(a.P, npx);
+    }
+    k_c_front<<<g, 256, 0, st>>>(a);
     const dim3 tiles((a.W + kCTX - 1) / kCTX, (a.H + kCTY - 1) / kCTY), tile_threads(kCTX, kCTY);
     k_c_var3<<<tiles, tile_threads, 0, st>>>(a);
     k_c_var4<<<g, 256, 0, st>>>(a);
-    k_c_var5<<<g, 256, 0, st>>>(a);
-    k_c_gauss1<<<g, 256, 0, st>>>(a);
-    k_c_gauss2<<<g, 256, 0, st>>>(a);
+    k_c_gauss<<<g, 256, 0, st>>>(a);
     kgk_vec *rin = a.R, *rout = a.R2;
     float4 *din = a.dm, *dout = a.dm2;
-    float *vin = a.var, *vout = var2;
+    int2 *vin = a.mv2, *vout = a.mv;
     for (int k = 0; k < repeats; ++k)
         for (int s = 0; s < stages; ++s) {
             const CompatIO io{rin, rout, din, dout, vin, vout};
@@ -658,8 +678,7 @@ kgk_status launch_compat(CompatArgs &a, float *var2, int repeats, int stages, cu
             std::swap(din, dout);
             std::swap(vin, vout);
         }
-    if (rin != a.R) k_copy_vec<<<g, 256, 0, st>>>(rin, a.R, (int)npx);
-    k_c_final<<<g, 256, 0, st>>>(a, vin);
+    k_c_final<<<g, 256, 0, st>>>(a, rin, vin);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "SVGF compat kernels");
@@ -679,8 +698,8 @@ kgk_status run_compat(kgk_vec *R, kgk_vec *F, kgk_svgf_buffer *P, kgk_svgf_buffe
     }
     CompatArgs a;
     a.W = W; a.H = H; a.frame = frame; a.R = R; a.F = F; a.P = P; a.C = C;
-    float *var2 = carve_compat(a, scratch, compat_fl(npx), compat_vec(npx));
-    const kgk_status stt = launch_compat(a, var2, repeats, stages, st);
+    carve_compat(a, scratch, compat_fl(npx), compat_vec(npx));
+    const kgk_status stt = launch_compat(a, repeats, stages, st);
     if (owned) dfree(owned);
     return stt;
 }
@@ -689,7 +708,6 @@ kgk_status run_compat(kgk_vec *R, kgk_vec *F, kgk_svgf_buffer *P, kgk_svgf_buffe
 // render.cuh:28 (init) and RayTrace.cuh:66-82 fill them.  A block builds its
 // 256 records in shared memory and writes them out as consecutive words, so
 // that the 112-byte records are stored with coalesced writes.
-constexpr int kRecWords = (int)(sizeof(kgk_svgf_buffer) / 4);
 __global__ void __launch_bounds__(256) k_gbuffer_to_records(const float4 *pos, const float4 *nrm, const float4 *alb,
                                                             const float4 *emi, size_t npx, kgk_svgf_buffer *C) {
     __shared__ __align__(16) unsigned s_rec[256 * kRecWords];
@@ -876,18 +894,6 @@ __global__ void k_s_temporal(StdArgs a) {
 // pixel for each distinct tap distance, and rl likewise; lg2(0) = -inf gives
 // w = 0 for normals facing away.  Both are the hardware approximations
 // (ex2.approx / lg2.approx, relative error ~2^-22).
-constexpr float kLog2e = 1.44269504088896341f;
-__device__ __forceinline__ float ex2a(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float lg2a(float x) {
-    float y;
-    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // Tiles of the standard filter's spatial passes: 32 x 8 pixels and a halo of
 // R pixels.  Entries outside the image carry material -2, which matches no
 // pixel, so taps need no bounds test.
@@ -1559,6 +1565,6 @@ extern "C" kgk_status kgk_svgf_apply_noalloc(kgk_vec *result, kgk_vec *filtered,
     a.W = W; a.H = H; a.frame = frame;
     a.R = result; a.F = filtered; a.P = prev; a.C = cur;
     // run_compat's layout, each array at its size for the largest image
-    float *var2 = carve_compat(a, base, compat_fl(kNaMax), compat_vec(kNaMax));
-    return launch_compat(a, var2, 5, 5, (cudaStream_t)cuda_stream);
+    carve_compat(a, base, compat_fl(kNaMax), compat_vec(kNaMax));
+    return launch_compat(a, 5, 5, (cudaStream_t)cuda_stream);
 }
