@@ -86,14 +86,14 @@ struct CompatArgs {
     int W, H, frame;
     kgk_vec *R, *F;
     kgk_svgf_buffer *P, *C;
-    float *M1, *M2, *sd, *gz, *s1, *s2, *sw;
+    float *M1, *M2, *sd, *gz;
     unsigned char *spatial;
     kgk_vec *R2;
     // The spatial passes' per-pixel guide, packed from the records: normal and
     // depth.
     float4 *gnd;
     // MaterialID and variance, the variance's sign bit set where ObjectID is -1
-    // (variances are never negative).  Before k_c_var4: ObjectID, MaterialID.
+    // (variances are never negative).  Before k_c_var: ObjectID, MaterialID.
     int2 *mv, *mv2;
     // the center pixel's albedo and willApplyATrousFilter (w = 1 or 0)
     float4 *galf;
@@ -101,8 +101,9 @@ struct CompatArgs {
     // luminance in w: written by the pass before (ping-pong), so a tap reads
     // it instead of dividing
     float4 *dm, *dm2;
-    // ColorHistory of the records while the passes run (over M1, M2, s1 and
-    // s2, whose last reader is k_c_var4)
+    // ColorHistory of the records while the passes run (over M1 and M2, whose
+    // last reader is k_c_var): written by every first stage for every pixel
+    // with an object
     kgk_vec *hist;
 };
 
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(256) k_c_init_prev(kgk_svgf_buffer *P, size_t 
 // (SVGF.cuh:50-98), the moments and the choice between their temporal update
 // and the spatial estimate (SVGF.cuh:114-165).  The records' moments of
 // SVGF.cuh:506-512 are not stored: every pixel's are replaced here or in
-// k_c_var4 before they are read.  At frame 0 the previous records hold no
+// k_c_var before they are read.  At frame 0 the previous records hold no
 // history and no samples, so they are not read.
 __global__ void k_c_front(CompatArgs a) {
     const int W = a.W, H = a.H;
@@ -229,9 +230,11 @@ __global__ void k_c_front(CompatArgs a) {
         const float d = c.Depth;
         a.gz[2 * p] = (a.C[W * y + x + dx].Depth - d) / (float)dx;
         a.gz[2 * p + 1] = (a.C[W * (y + dy) + x].Depth - d) / (float)dy;
-        // the guide k_c_var3 reads (the records as they are before k_c_var4)
+        // the guide k_c_var reads (the records as they are before it)
         a.gnd[p] = make_float4(c.Normal.x, c.Normal.y, c.Normal.z, d);
         a.mv[p] = make_int2(c.ObjectID, mat);
+        const float3 alb = v3(c.Albedo);
+        a.galf[p] = make_float4(alb.x, alb.y, alb.z, c.willApplyATrousFilter ? 1.0f : 0.0f);
     }
 }
 
@@ -243,11 +246,15 @@ __constant__ float cKW[25] = {1 / 256.0f, 4 / 256.0f, 6 / 256.0f, 4 / 256.0f, 1 
                               4 / 256.0f, 16 / 256.0f, 24 / 256.0f, 16 / 256.0f, 4 / 256.0f,
                               1 / 256.0f, 4 / 256.0f, 6 / 256.0f, 4 / 256.0f, 1 / 256.0f};
 
-// 7x7 edge-stopped moment filter (SVGF.cuh:166-225) on 32 x 8-pixel tiles:
-// a block stages the guide, ids and moments of its pixels and a halo of 3,
-// then sums in the reference's order (kx outer, ky inner).
+// The rest of VarianceEstimation (SVGF.cuh:166-275): the 7x7 edge-stopped
+// moment filter on 32 x 8-pixel tiles - a block stages the guide, ids and
+// moments of its pixels and a halo of 3, then sums in the reference's order
+// (kx outer, ky inner) - then the pixel's own record: without an object or an
+// estimate it is reset, the others get their moments.  The variance goes to
+// mv2 (the records take their final one in k_c_final); the guide of a reset
+// pixel stays as it was, no reader uses it.
 constexpr int kCTX = 32, kCTY = 8;
-__global__ void __launch_bounds__(256) k_c_var3(CompatArgs a) {
+__global__ void __launch_bounds__(256) k_c_var(CompatArgs a) {
     constexpr int R = 3, SX = kCTX + 2 * R, SY = kCTY + 2 * R;
     __shared__ float4 s_nd[SY * SX];
     __shared__ int2 s_om[SY * SX];
@@ -266,77 +273,61 @@ __global__ void __launch_bounds__(256) k_c_var3(CompatArgs a) {
     const int x = blockIdx.x * kCTX + threadIdx.x, y = blockIdx.y * kCTY + threadIdx.y;
     if (x >= W || y >= H) return;
     const int p = W * y + x, c = SX * (threadIdx.y + R) + threadIdx.x + R;
-    a.sw[p] = a.s1[p] = a.s2[p] = 0.0f;
-    if (!a.spatial[p]) return;
-    const float4 cn = s_nd[c];
-    const int cmat = s_om[c].y;
-    const float3 n = f3(cn);
-    const float gzx = a.gz[2 * p], gzy = a.gz[2 * p + 1];
-    float s1 = 0, s2 = 0, sw = 0;
-    for (int kx = -3; kx <= 3; ++kx) {
-        const int nx = x + kx;
-        if (nx < 0 || nx >= W) continue;
-        const float hx = cK7[kx + 3];
-        for (int ky = -3; ky <= 3; ++ky) {
-            const int ny = y + ky;
-            if (ny < 0 || ny >= H) continue;
-            const float hy = cK7[ky + 3];
-            if (kx == 0 && ky == 0) {
-                s1 += hx * hy * s_m[c].x;
-                s2 += hx * hy * s_m[c].y;
-                sw += hx * hy;
-                continue;
+    const int2 own = s_om[c];
+    const bool sp = a.spatial[p];
+    float m1 = s_m[c].x, m2 = s_m[c].y;
+    bool reset = own.x == -1;
+    if (sp && !reset) {
+        const float4 cn = s_nd[c];
+        const float3 n = f3(cn);
+        const float gzx = a.gz[2 * p], gzy = a.gz[2 * p + 1];
+        float s1 = 0, s2 = 0, sw = 0;
+        for (int kx = -3; kx <= 3; ++kx) {
+            const int nx = x + kx;
+            if (nx < 0 || nx >= W) continue;
+            const float hx = cK7[kx + 3];
+            for (int ky = -3; ky <= 3; ++ky) {
+                const int ny = y + ky;
+                if (ny < 0 || ny >= H) continue;
+                const float hy = cK7[ky + 3];
+                if (kx == 0 && ky == 0) {
+                    s1 += hx * hy * m1;
+                    s2 += hx * hy * m2;
+                    sw += hx * hy;
+                    continue;
+                }
+                const int t = c + SX * ky + kx;
+                const int2 om = s_om[t];
+                if (om.x == -1) continue;
+                const float4 qn = s_nd[t];
+                const float wm = own.y == om.y ? 1.0f : 0.0f;
+                const float wz = ex2a(depth_arg(cn.w, qn.w, (float)kx * gzx + (float)ky * gzy));
+                const float wn = normal_w(n, f3(qn));
+                const float w = hx * hy * wz * wn * wm;
+                s1 += w * s_m[t].x;
+                s2 += w * s_m[t].y;
+                sw += w;
             }
-            const int t = c + SX * ky + kx;
-            const int2 om = s_om[t];
-            if (om.x == -1) continue;
-            const float4 qn = s_nd[t];
-            const float wm = cmat == om.y ? 1.0f : 0.0f;
-            const float wz = ex2a(depth_arg(cn.w, qn.w, (float)kx * gzx + (float)ky * gzy));
-            const float wn = normal_w(n, f3(qn));
-            const float w = hx * hy * wz * wn * wm;
-            s1 += w * s_m[t].x;
-            s2 += w * s_m[t].y;
-            sw += w;
         }
+        reset = sw == 0.0f;
+        m1 = s1 / sw;
+        m2 = s2 / sw;
     }
-    a.s1[p] = s1;
-    a.s2[p] = s2;
-    a.sw[p] = sw;
-}
-
-// The rest of VarianceEstimation (SVGF.cuh:226-275): records without an object
-// or an estimate are reset, the others get their moments; the variance goes to
-// mv (the records take their final one in k_c_final).
-__global__ void k_c_var4(CompatArgs a) {
-    const int W = a.W;
-    FOR_PIXELS(W * a.H) {
-        kgk_svgf_buffer &c = a.C[p];
-        const int2 om = a.mv[p];
-        const bool sp = a.spatial[p];
-        const float sw = a.sw[p];
-        if (om.x == -1 || (sp && sw == 0.0f)) {
-            a.F[p] = a.R[p];
-            sb_init(c);
-            c.willApplyATrousFilter = false;
-            a.gnd[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            a.mv[p] = make_int2(-1, (int)0x80000000);
-            continue;
-        }
-        float m1, m2;
-        if (sp) {
-            m1 = a.s1[p] / sw;
-            m2 = a.s2[p] / sw;
-            c.MomentOne = m1;
-            c.MomentTwo = m2;
-            if (a.frame == 0 || c.PosLastFrameI[0] == -1) c.sampleNum = 1;
-            else c.sampleNum = a.P[W * c.PosLastFrameI[1] + c.PosLastFrameI[0]].sampleNum + 1;
-        } else {
-            m1 = a.M1[p];
-            m2 = a.M2[p];
-        }
-        a.mv[p] = make_int2(om.y, __float_as_int(fminf(fmaxf(0.0f, m2 - m1 * m1), 1000.0f)));
+    kgk_svgf_buffer &r = a.C[p];
+    if (reset) {
+        a.F[p] = a.R[p];
+        sb_init(r);
+        r.willApplyATrousFilter = false;
+        a.mv2[p] = make_int2(-1, (int)0x80000000);
+        return;
     }
+    if (sp) {
+        r.MomentOne = m1;
+        r.MomentTwo = m2;
+        if (a.frame == 0 || r.PosLastFrameI[0] == -1) r.sampleNum = 1;
+        else r.sampleNum = a.P[W * r.PosLastFrameI[1] + r.PosLastFrameI[0]].sampleNum + 1;
+    }
+    a.mv2[p] = make_int2(own.y, __float_as_int(fminf(fmaxf(0.0f, m2 - m1 * m1), 1000.0f)));
 }
 
 // ApplyGaussianFilterToVar (SVGF.cuh:277-344), and what the a-trous passes
@@ -355,42 +346,43 @@ __global__ void k_c_gauss(CompatArgs a) {
             for (int ky = -1; ky <= 1; ++ky) {
                 const int ny = y + ky;
                 if (ny < 0 || ny >= H) continue;
-                const int v = a.mv[W * ny + nx].y;
+                const int v = a.mv2[W * ny + nx].y;
                 if (v < 0) continue;
                 const float w = hx * cKG[ky + 1];
                 sv += w * __int_as_float(v);
                 sw += w;
             }
         }
-        kgk_svgf_buffer &c = a.C[p];
-        const int2 own = a.mv[p];
+        const int2 own = a.mv2[p];
+        const bool miss = own.y < 0;
         float var = __int_as_float(own.y & 0x7fffffff), sd = 0.0f;
-        bool filt = c.willApplyATrousFilter;
-        if (sw == 0.0f) {
-            c.MomentOne = -1.0f;
-            c.MomentTwo = -1.0f;
-            c.sampleNum = 0;
-        }
+        float4 af = a.galf[p];
+        if (miss) af = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // reset by k_c_var
         if (sv == 0.0f || sw == 0.0f) {
-            filt = false;
+            kgk_svgf_buffer &c = a.C[p];
+            if (sw == 0.0f) {
+                c.MomentOne = -1.0f;
+                c.MomentTwo = -1.0f;
+                c.sampleNum = 0;
+            }
+            af.w = 0.0f;
             c.willApplyATrousFilter = false;
         } else {
             var = sv / sw;
             sd = sqrtf(var);
         }
         a.sd[p] = sd;
-        a.mv2[p] = make_int2(own.x, __float_as_int(var) | (own.y & (int)0x80000000));
-        const float3 alb = v3(c.Albedo);
-        a.galf[p] = make_float4(alb.x, alb.y, alb.z, filt ? 1.0f : 0.0f);
-        const float3 dc = div3(v3(a.R[p]), alb + f3(kS, kS, kS));
+        a.mv[p] = make_int2(own.x, __float_as_int(var) | (own.y & (int)0x80000000));
+        a.galf[p] = af;
+        const float3 dc = div3(v3(a.R[p]), f3(af) + f3(kS, kS, kS));
         a.dm[p] = make_float4(dc.x, dc.y, dc.z, lumf(dc));
-        a.hist[p] = c.ColorHistory;
         // the a-trous passes' depth gradient (SVGF.cuh:366-372), from the
-        // records as k_c_var4 left them
+        // records as k_c_var left them: a reset one's depth is 0
         const int dx = x < W / 2 ? 1 : -1, dy = y < H / 2 ? 1 : -1;
-        const float d = a.gnd[p].w;
-        a.gz[2 * p] = (a.gnd[W * y + x + dx].w - d) / (float)dx;
-        a.gz[2 * p + 1] = (a.gnd[W * (y + dy) + x].w - d) / (float)dy;
+        const int qx = W * y + x + dx, qy = W * (y + dy) + x;
+        const float d = miss ? 0.0f : a.gnd[p].w;
+        a.gz[2 * p] = ((a.mv2[qx].y < 0 ? 0.0f : a.gnd[qx].w) - d) / (float)dx;
+        a.gz[2 * p + 1] = ((a.mv2[qy].y < 0 ? 0.0f : a.gnd[qy].w) - d) / (float)dy;
     }
 }
 
@@ -404,8 +396,9 @@ __global__ void k_c_gauss(CompatArgs a) {
 // Instruction issue bounds a pass (two IEEE divisions and two expf a tap
 // before, one reciprocal and one ex2 now), then shared memory (40 B a tap).
 // 1080p: a pass 202 / 195 / 201 / 247 / 244 us at steps 1 / 2 / 4 / 8 / 16 ->
-// 98 / 99 / 118 / 144 / 146; the call 6.35 -> 4.15 ms, with the front and
-// variance kernels' passes over the 112-byte records 1.19 -> 0.65 ms.  Error
+// 98 / 99 / 118 / 144 / 146, with two pixels a thread at the last two 123 /
+// 123; the passes over the 112-byte records before and after 1.19 -> 0.45 ms;
+// the call 6.47 -> 3.67 ms.  Error
 // against 64 bits over 64 x 64 to 2560 x 1440, with and without motion:
 // 3.6e-7 to 5.4e-7 before and after.
 struct CompatIO {
@@ -417,43 +410,44 @@ struct CompatIO {
     int2 *vout;
 };
 
-template <class Src>
-__device__ __forceinline__ void compat_atrous_px(const CompatArgs &a, const CompatIO &io, const Src &S, int x, int y,
-                                                 int stage) {
-    const int W = a.W, H = a.H, p = W * y + x, step = 1 << stage;
-    const float4 af = a.galf[p];
-    const float4 g = S.nd(0, 0);
-    const int2 om = S.mv(0, 0);
-    const float4 dcl = S.dm(0, 0);
-    const float l = dcl.w, d = g.w;
-    const float gx = a.gz[2 * p], gy = a.gz[2 * p + 1];
-    const float3 n = f3(g);
-    const bool filt = af.w != 0.0f;
-    // the luminance weight's factor of |l - nl| (0: no luminance weight)
-    const float rl = filt ? __fdividef(-kLog2e, 4.0f * a.sd[p] + kS) : 0.0f;
-    // a tap brighter than this is left out (SVGF.cuh:405-411, whose first two
-    // bounds compare in double)
-    const float bright = (double)l > 0.5 ? 5 * l : (double)l > 0.1 ? 50 * l : l > kS ? 100 * l : INFINITY;
-    const float cvar = __int_as_float(om.y & 0x7fffffff);
-    float3 srad = f3(0.0f, 0.0f, 0.0f);
-    float svar = 0.0f, swt = 0.0f;
-#pragma unroll
-    for (int ki = 0; ki < 25; ++ki) {
-        const float h = cKW[ki];
-        const int ox = (ki % 5 - 2) * step, oy = (ki / 5 - 2) * step;
-        if (ki == 12) {
-            svar += h * h * cvar;
-            srad += f3(dcl) * h;
-            swt += h;
-            continue;
-        }
-        const int qx = x + ox, qy = y + oy;
-        if (qx < 0 || qx >= W || qy < 0 || qy >= H) continue;
-        const int2 eo = S.mv(ox, oy);
-        const float4 em = S.dm(ox, oy);
-        if (eo.y < 0 || em.w > bright) continue;
-        const float4 eg = S.nd(ox, oy);
-        // absolute coordinates in the depth weight, SVGF.cuh:426
+// One pixel's part of a pass: what its taps need, and their sums.
+struct CompatPx {
+    int p;
+    float4 af, dcl;   // albedo and filter flag, own demodulated radiance
+    int2 om;          // own material and variance
+    float3 n;
+    float d, l, gx, gy;
+    float rl;         // the luminance weight's factor of |l - nl| (0: no luminance weight)
+    float bright;     // a tap brighter than this is left out
+    float3 srad;
+    float svar, swt;
+
+    __device__ __forceinline__ float var() const { return __int_as_float(om.y & 0x7fffffff); }
+    __device__ __forceinline__ void start(const CompatArgs &a, int p_, float4 nd, float4 dm, int2 mv) {
+        p = p_;
+        af = a.galf[p];
+        dcl = dm;
+        om = mv;
+        n = f3(nd);
+        d = nd.w;
+        l = dm.w;
+        const float2 g = reinterpret_cast<const float2 *>(a.gz)[p];
+        gx = g.x;
+        gy = g.y;
+        rl = af.w != 0.0f ? __fdividef(-kLog2e, 4.0f * a.sd[p] + kS) : 0.0f;
+        // SVGF.cuh:405-411, whose first two bounds compare in double
+        bright = (double)l > 0.5 ? 5 * l : (double)l > 0.1 ? 50 * l : l > kS ? 100 * l : INFINITY;
+        srad = f3(0.0f, 0.0f, 0.0f);
+        svar = swt = 0.0f;
+    }
+    __device__ __forceinline__ void center(float h) {
+        svar += h * h * var();
+        srad += f3(dcl) * h;
+        swt += h;
+    }
+    // a neighbour at (qx, qy); absolute coordinates in the depth weight, SVGF.cuh:426
+    __device__ __forceinline__ void tap(float h, int qx, int qy, int2 eo, float4 em, float4 eg) {
+        if (eo.y < 0 || em.w > bright) return;
         const float e = depth_arg(d, eg.w, (float)qx * gx + (float)qy * gy) + fminf(fabsf(l - em.w), 3e38f) * rl;
         float w = h * ex2a(e) * normal_w(n, f3(eg));
         w = om.x == eo.x ? w : 0.0f;
@@ -461,23 +455,79 @@ __device__ __forceinline__ void compat_atrous_px(const CompatArgs &a, const Comp
         svar += w * w * __int_as_float(eo.y);
         swt += w;
     }
-    const kgk_vec rin = io.Rin[p];
-    if (om.y < 0 || swt < 1e-6f || swt * swt < 1e-6f) {
-        io.Rout[p] = rin;
-        io.vout[p] = om;
-        io.dmout[p] = dcl;
-        return;
+    __device__ __forceinline__ void finish(const CompatArgs &a, const CompatIO &io, int stage) const {
+        const kgk_vec rin = io.Rin[p];
+        if (om.y < 0 || swt < 1e-6f || swt * swt < 1e-6f) {
+            io.Rout[p] = rin;
+            io.vout[p] = om;
+            io.dmout[p] = dcl;
+            return;
+        }
+        const float3 alb = f3(af);
+        const float3 fl = srad / swt;
+        const float fv = svar / (swt * swt);
+        const float cw = 0.2f;
+        const float3 o = (fl * alb) * cw + v3(rin) * (1 - cw);
+        io.Rout[p] = kv(o);
+        const float3 od = div3(o, alb + f3(kS, kS, kS));
+        io.dmout[p] = make_float4(od.x, od.y, od.z, lumf(od));
+        io.vout[p] = make_int2(om.x, __float_as_int(af.w != 0.0f ? cw * var() + (1 - cw) * fv : var()));
+        if (stage == 0) a.hist[p] = kv(o);
     }
-    const float3 alb = f3(af);
-    const float3 fl = srad / swt;
-    const float fv = svar / (swt * swt);
-    const float cw = 0.2f;
-    const float3 o = (fl * alb) * cw + v3(rin) * (1 - cw);
-    io.Rout[p] = kv(o);
-    const float3 od = div3(o, alb + f3(kS, kS, kS));
-    io.dmout[p] = make_float4(od.x, od.y, od.z, lumf(od));
-    io.vout[p] = make_int2(om.x, __float_as_int(filt ? cw * cvar + (1 - cw) * fv : cvar));
-    if (stage == 0) a.hist[p] = kv(o);
+};
+
+template <class Src>
+__device__ __forceinline__ void compat_atrous_px(const CompatArgs &a, const CompatIO &io, const Src &S, int x, int y,
+                                                 int stage) {
+    const int W = a.W, H = a.H, step = 1 << stage;
+    CompatPx A;
+    A.start(a, W * y + x, S.nd(0, 0), S.dm(0, 0), S.mv(0, 0));
+#pragma unroll
+    for (int ki = 0; ki < 25; ++ki) {
+        const int ox = (ki % 5 - 2) * step, oy = (ki / 5 - 2) * step;
+        if (ki == 12) {
+            A.center(cKW[ki]);
+            continue;
+        }
+        const int qx = x + ox, qy = y + oy;
+        if (qx < 0 || qx >= W || qy < 0 || qy >= H) continue;
+        A.tap(cKW[ki], qx, qy, S.mv(ox, oy), S.dm(ox, oy), S.nd(ox, oy));
+    }
+    A.finish(a, io, stage);
+}
+
+// Two pixels of a column, `step` rows apart: four of the five tap rows are the
+// same, so 30 neighbours are read for both where 50 would be.  Each pixel's
+// taps keep their order.  B (the lower one) may lie outside the image.
+template <class Src>
+__device__ __forceinline__ void compat_atrous_px2(const CompatArgs &a, const CompatIO &io, const Src &S, int x, int y,
+                                                  int stage) {
+    const int W = a.W, H = a.H, step = 1 << stage;
+    const bool two = y + step < H;
+    CompatPx A, B;
+    A.start(a, W * y + x, S.nd(0, 0), S.dm(0, 0), S.mv(0, 0));
+    if (two) B.start(a, W * (y + step) + x, S.nd(0, step), S.dm(0, step), S.mv(0, step));
+    else B = A;
+#pragma unroll
+    for (int r = 0; r < 6; ++r)
+#pragma unroll
+        for (int c = 0; c < 5; ++c) {
+            const int ox = (c - 2) * step, oy = (r - 2) * step;
+            const int qx = x + ox, qy = y + oy;
+            if (qx < 0 || qx >= W || qy < 0 || qy >= H) continue;
+            const int2 eo = S.mv(ox, oy);
+            const float4 em = S.dm(ox, oy), eg = S.nd(ox, oy);
+            if (r < 5) {
+                if (r == 2 && c == 2) A.center(cKW[12]);
+                else A.tap(cKW[r * 5 + c], qx, qy, eo, em, eg);
+            }
+            if (r > 0) {
+                if (r == 3 && c == 2) B.center(cKW[12]);
+                else B.tap(cKW[(r - 1) * 5 + c], qx, qy, eo, em, eg);
+            }
+        }
+    A.finish(a, io, stage);
+    if (two) B.finish(a, io, stage);
 }
 
 // Taps read straight from the global arrays (offsets from pixel p).
@@ -499,10 +549,11 @@ __global__ void k_c_atrous(CompatArgs a, CompatIO io, int stage) {
 }
 
 // The same stage for steps 1, 2 and 4 on 32 x 8-pixel tiles: a block stages
-// its pixels and a halo of 2 * step (all 25 taps and the depth gradient's
-// neighbours) in shared memory - guide, ids, demodulated radiance, variance -
-// then filters from there.  Entries outside the image are never read (the
-// tap's bounds test comes first).
+// its pixels and a halo of 2 * step in shared memory - guide, demodulated
+// radiance, material and variance - then filters from there.  Entries outside
+// the image are never read (the tap's bounds test comes first).  Two pixels a
+// thread, as in the rows below, measured slower here (98 / 99 / 118 us a pass
+// to 110 / 113 / 122: half the blocks, 76 registers, for little less staging).
 template <int kStep> struct CTile {
     static constexpr int R = 2 * kStep, SX = kCTX + 2 * R, SY = kCTY + 2 * R, N = SX * SY;
     static constexpr size_t kSmem = (size_t)N * (2 * sizeof(float4) + sizeof(int2));
@@ -542,16 +593,19 @@ __global__ void __launch_bounds__(256) k_c_atrous_tile(CompatArgs a, CompatIO io
     compat_atrous_px(a, io, S, x, y, kStep == 1 ? 0 : kStep == 2 ? 1 : 2);
 }
 
-// The same stage for steps of 8 and more on row segments: a block of 256
-// threads takes 256 pixels of one row and stages the five rows its taps read
-// (y + {-2, -1, 0, 1, 2} step), each 256 + 4 step entries wide, so that every
-// tap comes from shared memory and the staging reads are coalesced.
+// The same stage for steps of 8 and more on row segments: a block of kRowT
+// threads takes kRowT pixels of two rows, step apart, and stages the six rows
+// their taps read, each kRowT + 4 step entries wide, so that every tap comes
+// from shared memory and the staging reads are coalesced (one row a block, 10
+// staged rows for what takes 6 here: 144 -> 125 us a pass at step 8, 146 ->
+// 124 at 16, 1080p; blocks of 128 and 192: the call 4.42 and 4.28 ms to 4.18).
+constexpr int kRowT = 256;
 template <int kStep> struct CRows {
-    static constexpr int T = 256, R = 2 * kStep, SX = T + 2 * R, N = 5 * SX;
+    static constexpr int T = kRowT, R = 2 * kStep, SX = T + 2 * R, N = 6 * SX;
     static constexpr size_t kSmem = (size_t)N * (2 * sizeof(float4) + sizeof(int2));
 };
 
-// Taps read from the five staged rows (row pitch SX, one row per step).
+// Taps read from the six staged rows (row pitch SX, one row per step).
 template <int SX, int kStep> struct CompatRows {
     const float4 *snd, *sdm;
     const int2 *smv;
@@ -562,14 +616,18 @@ template <int SX, int kStep> struct CompatRows {
     __device__ float4 dm(int ox, int oy) const { return sdm[at(ox, oy)]; }
 };
 
+// Blocks along y: one per pair of rows (y, y + step).
+__host__ __device__ constexpr int row_pairs(int H, int step) { return (H + 2 * step - 1) / (2 * step) * step; }
+
 template <int kStep>
-__global__ void __launch_bounds__(256) k_c_atrous_rows(CompatArgs a, CompatIO io) {
+__global__ void __launch_bounds__(kRowT) k_c_atrous_rows(CompatArgs a, CompatIO io) {
     using T = CRows<kStep>;
     extern __shared__ __align__(16) unsigned char smem[];
     float4 *s_nd = (float4 *)smem;
     float4 *s_dm = s_nd + T::N;
     int2 *s_mv = (int2 *)(s_dm + T::N);
-    const int W = a.W, H = a.H, y = blockIdx.y;
+    const int W = a.W, H = a.H, y = (int)blockIdx.y / kStep * (2 * kStep) + (int)blockIdx.y % kStep;
+    if (y >= H) return;  // the whole block: its pair lies below the image
     const int x0 = blockIdx.x * T::T - T::R;
     for (int i = threadIdx.x; i < T::N; i += T::T) {
         const int gx = x0 + i % T::SX, gy = y + (i / T::SX - 2) * kStep;
@@ -585,18 +643,19 @@ __global__ void __launch_bounds__(256) k_c_atrous_rows(CompatArgs a, CompatIO io
     constexpr int stage = kStep == 8 ? 3 : kStep == 16 ? 4 : kStep == 32 ? 5 : 6;
     static_assert((1 << stage) == kStep, "row-tile steps are 8, 16, 32 and 64");
     const CompatRows<T::SX, kStep> S{s_nd, s_dm, s_mv, 2 * T::SX + (int)threadIdx.x + T::R};
-    compat_atrous_px(a, io, S, x, y, stage);
+    compat_atrous_px2(a, io, S, x, y, stage);
 }
 
 // The records, the result and the filtered image after the last pass (its
-// output radiance Rl): pixels without an object keep the image k_c_var4 gave
-// them.
+// output radiance Rl): pixels without an object keep the image k_c_var gave
+// them and an empty history.
 __global__ void k_c_final(CompatArgs a, const kgk_vec *Rl, const int2 *mv) {
     FOR_PIXELS(a.W * a.H) {
         const int v = mv[p].y;
         kgk_svgf_buffer &c = a.C[p];
-        const kgk_vec h = a.hist[p];
+        kgk_vec h = {0, 0, 0, 0};
         if (v >= 0) {
+            h = a.hist[p];
             a.F[p] = Rl[p];
             c.willApplyTemporalAccumulation = true;
         }
@@ -606,28 +665,24 @@ __global__ void k_c_final(CompatArgs a, const kgk_vec *Rl, const int2 *mv) {
     }
 }
 
-// Scratch of the compat pipeline, carved from one block: M1, M2, s1, s2 (then
-// hist over these four), sd, gz (two arrays), sw at `fl` bytes each, then R2
-// (`vec` bytes), the guide (gnd, 16 B a pixel), the two demodulated radiance
-// buffers (dm, dm2, 16 B each), albedo + filter flag (galf, 16 B), material +
-// variance twice (mv, mv2, 8 B each), then the per-pixel spatial flags; every
-// array starts on a 256-byte boundary.
+// Scratch of the compat pipeline, carved from one block: hist (`vec` bytes; M1
+// and M2, `fl` bytes each, lie over it), R2, the guide (gnd, 16 B a pixel), the
+// two demodulated radiance buffers (dm, dm2, 16 B each), albedo + filter flag
+// (galf, 16 B), material + variance twice (mv, mv2, 8 B each), sd, gz (two
+// arrays), then the per-pixel spatial flags; every array starts on a 256-byte
+// boundary.
 constexpr size_t scratch_up(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr size_t compat_fl(size_t npx) { return scratch_up(npx * sizeof(float)); }
 constexpr size_t compat_vec(size_t npx) { return scratch_up(npx * sizeof(kgk_vec)); }
 constexpr size_t compat_scratch_bytes(size_t npx) {
-    return 8 * compat_fl(npx) + 5 * compat_vec(npx) + 2 * scratch_up(npx * sizeof(int2)) + npx;
+    return 3 * compat_fl(npx) + std::max(compat_vec(npx), 2 * compat_fl(npx)) + 5 * compat_vec(npx) + 2 * scratch_up(npx * sizeof(int2)) + npx;
 }
 
 void carve_compat(CompatArgs &a, unsigned char *b, size_t fl, size_t vec) {
-    a.hist = (kgk_vec *)b;  // 4 fl >= vec
-    a.M1 = (float *)b; b += fl;
-    a.M2 = (float *)b; b += fl;
-    a.s1 = (float *)b; b += fl;
-    a.s2 = (float *)b; b += fl;
-    a.sd = (float *)b; b += fl;
-    a.gz = (float *)b; b += 2 * fl;
-    a.sw = (float *)b; b += fl;
+    a.hist = (kgk_vec *)b;
+    a.M1 = (float *)b;
+    a.M2 = (float *)(b + fl);
+    b += std::max(vec, 2 * fl);
     a.R2 = (kgk_vec *)b; b += vec;
     a.gnd = (float4 *)b; b += vec;
     a.dm = (float4 *)b; b += vec;
@@ -635,6 +690,8 @@ void carve_compat(CompatArgs &a, unsigned char *b, size_t fl, size_t vec) {
     a.galf = (float4 *)b; b += vec;
     a.mv = (int2 *)b; b += scratch_up(vec / 2);
     a.mv2 = (int2 *)b; b += scratch_up(vec / 2);
+    a.sd = (float *)b; b += fl;
+    a.gz = (float *)b; b += 2 * fl;
     a.spatial = b;
 }
 
@@ -656,22 +713,21 @@ kgk_status launch_compat(CompatArgs &a, int repeats, int stages, cudaStream_t st
     }
     k_c_front<<<g, 256, 0, st>>>(a);
     const dim3 tiles((a.W + kCTX - 1) / kCTX, (a.H + kCTY - 1) / kCTY), tile_threads(kCTX, kCTY);
-    k_c_var3<<<tiles, tile_threads, 0, st>>>(a);
-    k_c_var4<<<g, 256, 0, st>>>(a);
+    k_c_var<<<tiles, tile_threads, 0, st>>>(a);
     k_c_gauss<<<g, 256, 0, st>>>(a);
     kgk_vec *rin = a.R, *rout = a.R2;
     float4 *din = a.dm, *dout = a.dm2;
-    int2 *vin = a.mv2, *vout = a.mv;
+    int2 *vin = a.mv, *vout = a.mv2;
     for (int k = 0; k < repeats; ++k)
         for (int s = 0; s < stages; ++s) {
             const CompatIO io{rin, rout, din, dout, vin, vout};
-            const dim3 rows((a.W + 255) / 256, a.H);
+            const dim3 rows8((a.W + kRowT - 1) / kRowT, row_pairs(a.H, 8)), rows16(rows8.x, row_pairs(a.H, 16));
             switch (s) {
                 case 0: k_c_atrous_tile<1><<<tiles, tile_threads, CTile<1>::kSmem, st>>>(a, io); break;
                 case 1: k_c_atrous_tile<2><<<tiles, tile_threads, CTile<2>::kSmem, st>>>(a, io); break;
                 case 2: k_c_atrous_tile<4><<<tiles, tile_threads, CTile<4>::kSmem, st>>>(a, io); break;
-                case 3: k_c_atrous_rows<8><<<rows, 256, CRows<8>::kSmem, st>>>(a, io); break;
-                case 4: k_c_atrous_rows<16><<<rows, 256, CRows<16>::kSmem, st>>>(a, io); break;
+                case 3: k_c_atrous_rows<8><<<rows8, kRowT, CRows<8>::kSmem, st>>>(a, io); break;
+                case 4: k_c_atrous_rows<16><<<rows16, kRowT, CRows<16>::kSmem, st>>>(a, io); break;
                 default: k_c_atrous<<<g, 256, 0, st>>>(a, io, s); break;
             }
             std::swap(rin, rout);
@@ -1506,7 +1562,7 @@ void kgk_host_free(void *p) {
 // must not allocate because cudaMalloc / cudaFree synchronise the whole device
 // and stall the caller's other streams.  This entry point takes its scratch
 // from g_svgf_scratch, a file-scope device array sized for
-// KGK_SVGF_NOALLOC_MAX_PIXELS pixels (129 B per pixel, ~34 MB); every GPU that
+// KGK_SVGF_NOALLOC_MAX_PIXELS pixels (125 B per pixel, ~33 MB); every GPU that
 // loads the library holds that array until the process exits.
 // ---------------------------------------------------------------------------
 #include <mutex>
