@@ -51,6 +51,23 @@ __device__ __forceinline__ void sincospi_feature(float x, float *s, float *c) {
     __sincosf(r * 3.14159265358979f, s, c);
 }
 
+// Features 2 i and 2 i + 1 of a raw query, packed (see encode_row).
+__device__ __forceinline__ uint32_t encode_pair(const float *raw, int i) {
+    if (i < 18) {
+        float s, co;
+        sincospi_feature(raw[i / 6] * (float)(1 << (i % 6)), &s, &co);
+        return pack2(s, co);
+    }
+    if (i < 21) return pack2(raw[3 + 2 * (i - 18)], raw[4 + 2 * (i - 18)]);
+    if (i < 27) {
+        float s, co;
+        sincospi_feature(raw[3 + i - 21], &s, &co);
+        return pack2(s, co);
+    }
+    if (i < 29) return pack2(raw[9 + 2 * (i - 27)], raw[10 + 2 * (i - 27)]);
+    return pack2(1.0f, 1.0f);
+}
+
 // All 64 input features of a raw query: 3 x 12 sine / cosine features of the
 // normalised position (6 octaves), normal and view direction, their sines and
 // cosines (12), roughness and albedo, six constant ones (the biases).
@@ -81,23 +98,21 @@ __device__ __forceinline__ void encode_row(const float *raw, float (&f)[64]) {
 }
 
 // ---------------------------------------------------------------------------
-// inference on the 5th-generation tensor cores (tcgen05 + TMEM)
+// The network on the 5th-generation tensor cores (tcgen05 + TMEM)
 //
 // A CTA holds the weights once (BF16, 128-byte-swizzled K-major, in shared
-// memory; each layer as K sub-tiles of 64 inputs) for its warpgroups, each
-// carrying its own tiles of 128 queries through the network: thread r of a
-// warpgroup owns row r.  Per layer a warpgroup writes the BF16 activations
-// (128 x W) to its shared-memory tile in the same layout, one elected thread
-// issues the tcgen05.mma (M=128, N=W, K=16 each) into the warpgroup's
-// 128 x W FP32 accumulator in tensor memory and commits to the warpgroup's
-// mbarrier; the threads then read their row back (tcgen05.ld 32x32b) and
+// memory; each layer as K sub-tiles of 64 inputs).  A tile is 128 samples:
+// thread r of its warpgroup owns row r, which is tensor-memory lane r.  Per
+// layer one elected thread issues the tcgen05.mma (M=128, N=W, K=16 each) into
+// the tile's 128 x W FP32 accumulator in tensor memory and commits to the
+// tile's mbarrier; the threads then read their row back (tcgen05.ld 32x32b) and
 // apply the ReLU and the BF16 rounding for the next layer in one conversion.
-// The warpgroups synchronise on their own named barriers, so the CUDA-core
-// work of one overlaps the MMAs of another.  Width 64: four warpgroups per
-// CTA, two CTAs per SM; width 128: two warpgroups, one CTA per SM (shared
-// memory).  The output layer uses N=16 (3 live rows of the padded weights).
-// Every wait is bounded: on a timeout the CTA raises *err, stops issuing and
-// frees its tensor memory.
+// Inference (k_infer_tc) keeps the activations in tensor memory, training
+// (k_train_fb_tc) in shared memory, from where they also go to its scratch.
+// Tiles synchronise on their own named barriers, so the CUDA-core work of one
+// overlaps the MMAs of another.  The output layer uses N=16 (3 live rows of the
+// padded weights).  Every wait is bounded: on a timeout the CTA raises *err,
+// stops issuing and frees its tensor memory.
 // ---------------------------------------------------------------------------
 namespace tc {
 
@@ -122,15 +137,9 @@ struct Tc {
     static constexpr uint32_t kSlotOff = kBarOff + 8 * kGroups;
     static constexpr uint32_t kSmemBytes = kSlotOff + 8 + 1024;     // + room to align the base to 1024 B
     static constexpr uint32_t kTmemCols = (uint32_t)W * kGroups;    // a W-column accumulator per warpgroup
-    // inference: two accumulators per warpgroup when a layer has two K
-    // sub-tiles, so the next layer's MMAs on the first sub-tile run while the
-    // second is converted
-    static constexpr int kAccBufs = kKSubs > 1 ? 2 : 1;
-    static constexpr uint32_t kInferTmemCols = kTmemCols * kAccBufs;
     static_assert(kAOff % 1024 == 0, "swizzle atoms need 1024-byte alignment");
     static_assert(kSmemBytes <= 227 * 1024, "shared memory per CTA");
     static_assert(kTmemCols * kCtasPerSm <= 512, "tensor memory per SM");
-    static_assert(kInferTmemCols * kCtasPerSm <= 512, "tensor memory per SM (inference)");
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -240,21 +249,107 @@ __device__ __forceinline__ bool wg_sync_or(int id, bool v) {
     return r != 0;
 }
 
+// Inference keeps the activations in tensor memory: a warpgroup's 128 x W
+// accumulator is read back, rounded and stored as the next layer's A operand
+// (W / 2 columns of BF16 pairs) beside it, and the MMA takes A from there.  In
+// shared memory the activations were written and read back by every layer
+// (width 64: 16 + 16 KB to 8 KB of weights), and that traffic, at 128 B a clock,
+// bound the kernel.  Shared memory now holds the weights alone, so one CTA per
+// SM carries as many tiles as the 512 columns take: four at width 64, two at
+// 128.  With tensor memory setting the tiles in flight, latency is what is
+// left: the next tile's features are made while the hidden layers' MMAs run,
+// and at width 128 a tile has two warpgroups, each converting half of the
+// columns of every row (tensor memory is reached by lane quarter, so warps w
+// and w + 4 share one).  Width 128: 824 -> 1160 TFLOP/s (a 4K frame's queries
+// 240 -> 169 us; one warpgroup a tile 183).  Width 64, 2^21 queries: 107 ->
+// 102 us (five tiles without the overlapped encoding 110, two warpgroups a tile
+// 106); leaving out the encoding, three of four MMAs or the query loads there
+// takes 8 % each: no one of them bounds it, four tiles' latency does.
+namespace tc {
 template <int W>
-__global__ void __launch_bounds__(128 * tc::Tc<W>::kGroups) k_infer_tc(const unsigned short *__restrict__ img,
-                                                                       const float *__restrict__ raw,
-                                                                       int stride_floats, int n, const int *n_dev,
-                                                                       float *out, float4 *rad, int *err) {
+struct Ti {
+    using T = Tc<W>;
+    static constexpr int kGroups = W == 64 ? 4 : 2;  // tiles in flight
+    static constexpr int kSplit = W == 64 ? 1 : 2;   // warpgroups per tile
+    static constexpr int kTileThreads = 128 * kSplit;
+    static constexpr uint32_t kBarOff = T::kAOff;  // past the weights
+    static constexpr uint32_t kSlotOff = kBarOff + 8 * kGroups;
+    static constexpr uint32_t kSmemBytes = kSlotOff + 8 + 1024;  // + room to align the base to 1024 B
+    // accumulator, then the A operand of the hidden layers, then of the first
+    static constexpr uint32_t kGroupCols = W + W / 2 + 32;
+    static constexpr uint32_t kCols = 512;
+    static_assert(kGroupCols * kGroups <= kCols, "tensor memory per SM");
+};
+
+// A from tensor memory (128 lanes, 8 columns of BF16 pairs per K = 16 step).
+__device__ __forceinline__ void mma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t b, uint32_t idesc,
+                                            uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(b), "r"(idesc), "r"(acc));
+}
+// 32 consecutive 32-bit columns of this thread's tensor-memory lane.
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
+        "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
+            taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
+                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+}  // namespace tc
+
+// Named barrier of the N threads of one tile, and its OR reduction.
+template <int N>
+__device__ __forceinline__ void tile_sync(int id) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory");
+}
+template <int N>
+__device__ __forceinline__ bool tile_sync_or(int id, bool v) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, %2, %3, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(r)
+        : "r"((uint32_t)v), "r"(id), "n"(N)
+        : "memory");
+    return r != 0;
+}
+
+template <int W>
+__global__ void __launch_bounds__(tc::Ti<W>::kTileThreads * tc::Ti<W>::kGroups, 1)
+    k_infer_tc(const unsigned short *__restrict__ img, const float *__restrict__ raw, int stride_floats, int n,
+               const int *n_dev, float *out, float4 *rad, int *err) {
     using namespace tc;
     using T = Tc<W>;
-    constexpr int kG = T::kGroups, P = Net<W>::kPitch;
+    using I = Ti<W>;
+    constexpr int kG = I::kGroups, P = Net<W>::kPitch;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;
     unsigned char *sm = smem_raw + pad;
     const uint32_t s0 = smem_u32(sm);
     const int tid = threadIdx.x, warp = tid >> 5;
-    const int g = tid >> 7, r = tid & 127;  // warpgroup, row
-    const int wgbar = 1 + g;                // its named barrier
+    const int g = tid / I::kTileThreads, r = tid & 127;  // tile slot, row
+    const int part = (tid >> 7) % I::kSplit;             // the part of the columns this thread converts
+    const bool first = part == 0 && r == 0;              // issues the tile's MMAs
+    const int tbar = 1 + g;                              // the tile's named barrier
     // weights: BF16 image rows (pitch P) -> swizzled K-major sub-tiles
     constexpr int kChunks = W / 8;  // 16-byte chunks of a W-input row
     for (int i = tid; i < (kLayers * W + kOutRows) * kChunks; i += blockDim.x) {
@@ -269,14 +364,14 @@ __global__ void __launch_bounds__(128 * tc::Tc<W>::kGroups) k_infer_tc(const uns
         }
         *reinterpret_cast<uint4 *>(sm + dst) = *reinterpret_cast<const uint4 *>(img + (size_t)row * P + c * 8);
     }
-    const uint32_t bar = s0 + T::kBarOff + 8u * (uint32_t)g;
-    if (r == 0) {
+    const uint32_t bar = s0 + I::kBarOff + 8u * (uint32_t)g;
+    if (first) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s0 + T::kSlotOff),
-                     "r"(T::kInferTmemCols)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s0 + I::kSlotOff),
+                     "r"(I::kCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -284,117 +379,120 @@ __global__ void __launch_bounds__(128 * tc::Tc<W>::kGroups) k_infer_tc(const uns
     fence_before();
     __syncthreads();
     fence_after();
-    constexpr uint32_t kGroupCols = (uint32_t)W * T::kAccBufs;
-    const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(sm + T::kSlotOff) + kGroupCols * (uint32_t)g;
-    const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's 32 TMEM lanes
+    const uint32_t base = *reinterpret_cast<volatile uint32_t *>(sm + I::kSlotOff);
+    const uint32_t tmem = base + I::kGroupCols * (uint32_t)g;          // accumulator
+    const uint32_t tmem_a = tmem + (uint32_t)W;                        // A operand of layers 1..
+    const uint32_t tmem_f = tmem_a + (uint32_t)W / 2;                  // features: A operand of layer 0
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;          // this warp's 32 lanes
     const int total = n_dev ? min(*n_dev, n) : n;
     uint32_t phase = 0;
-    bool failed = false;
-    unsigned char *A = sm + T::kAOff + (uint32_t)g * T::kATile;
-    const uint32_t a_addr = s0 + T::kAOff + (uint32_t)g * T::kATile;
-    for (int tile = blockIdx.x * kG + g; tile * kRows < total; tile += gridDim.x * kG) {
+    bool failed = false, ok = true;
+    const uint64_t bdesc = sw128_desc(s0);  // + offsets in 16 B units
+    // the MMAs of layer l, issued once every row's A is stored
+    auto issue = [&](int l) {
+        const bool last = l == kLayers;
+        const uint32_t boff = last ? T::kOutOff : T::layer_off(l);
+        const uint32_t bsub = last ? kOutSub : T::kWSub;
+        const uint32_t id = last ? idesc_bf16(128, 16) : idesc_bf16(128, W);
+        const uint32_t ta = l == 0 ? tmem_f : tmem_a;
+        constexpr int kMax = W / 16;
+#pragma unroll
+        for (int kk = 0; kk < kMax; ++kk) {
+            if (kk >= Net<W>::in(l) / 16) break;
+            const uint32_t j = (uint32_t)kk >> 2;  // sub-tile; 32 B steps inside
+            mma_bf16_ta(tmem, ta + 8u * (uint32_t)kk, bdesc + ((boff + j * bsub) >> 4) + 2u * (uint32_t)(kk & 3), id,
+                        kk > 0 ? 1u : 0u);
+        }
+        commit(bar);
+    };
+    // A is stored (by every row: the barrier) -> layer l's MMAs
+    auto stored = [&](int l) {
+        if (l > 0) {  // layer 0's barrier is the tile's own, below
+            tmem_wait_st();
+            fence_before();
+            tile_sync<I::kTileThreads>(tbar);
+        }
+        if (first) {
+            fence_after();
+            issue(l);
+        }
+    };
+    float rw[kRaw];
+    auto load_raw = [&](int q) {
+#pragma unroll
+        for (int k = 0; k < kRaw; ++k) rw[k] = q < total ? raw[(size_t)q * stride_floats + k] : 0.0f;
+    };
+    // a quarter of the features of the query in rw
+    auto encode = [&](int c) {
+        uint32_t h[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) h[i] = encode_pair(rw, 8 * c + i);
+        tmem_st8(tmem_f + lanes + 8u * (uint32_t)c, h);
+    };
+    // this thread's share of the features, quarter k of four: all of it, or
+    // quarters 0 and 3 / 1 and 2 of the two warpgroups (11 and 13 of the 24
+    // sine / cosine pairs)
+    auto encode_own = [&](int k) {
+        if (I::kSplit == 1) encode(k);
+        else if ((part == 0) == (k == 0 || k == 3)) encode(k);
+    };
+    const int stride = gridDim.x * kG;
+    int tile = blockIdx.x * kG + g;
+    if (tile * kRows < total) {
+        load_raw(tile * kRows + r);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) encode_own(k);
+    }
+    for (; tile * kRows < total; tile += stride) {
         const int q = tile * kRows + r;
         const bool live = q < total;
-        // input encoding of row r (the first K sub-tile)
-        {
-            float rw[kRaw];
-#pragma unroll
-            for (int k = 0; k < kRaw; ++k) rw[k] = live ? raw[(size_t)q * stride_floats + k] : 0.0f;
-            float f[64];
-            encode_row(rw, f);
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                uint4 v;
-                v.x = pack2(f[8 * c + 0], f[8 * c + 1]);
-                v.y = pack2(f[8 * c + 2], f[8 * c + 3]);
-                v.z = pack2(f[8 * c + 4], f[8 * c + 5]);
-                v.w = pack2(f[8 * c + 6], f[8 * c + 7]);
-                *reinterpret_cast<uint4 *>(A + sw_off(r, c)) = v;
-            }
-        }
-        float y[3] = {0.0f, 0.0f, 0.0f};
-        // the MMAs of layer l on K sub-tile h (k-steps 4h .. 4h + 3) into the
-        // layer's accumulator; issued by row 0 once the sub-tile is written
-        auto issue = [&](int l, int h) {
-            const bool last = l == kLayers;
-            const uint32_t boff = last ? T::kOutOff : T::layer_off(l);
-            const uint32_t bsub = last ? kOutSub : T::kWSub;
-            const uint32_t id = last ? idesc_bf16(128, 16) : idesc_bf16(128, W);
-            const uint32_t d = tmem + (uint32_t)W * (uint32_t)(l % T::kAccBufs);
-            const int nk = Net<W>::in(l) / 16;
-            for (int kk = 4 * h; kk < nk && kk < 4 * h + 4; ++kk) {
-                const uint32_t j = (uint32_t)kk >> 2, o = 2u * (uint32_t)(kk & 3);  // sub-tile, 32 B steps
-                mma_bf16(d, sw128_desc(a_addr + j * kSub) + o, sw128_desc(s0 + boff + j * bsub) + o, id,
-                         kk > 0 ? 1u : 0u);
-            }
-        };
-        fence_async_smem();
+        // the barrier before layer 0 tells all of the tile's threads whether a
+        // wait timed out in any of them (inside a tile they go on: every wait
+        // is bounded)
+        tmem_wait_st();
         fence_before();
-        wg_sync(wgbar);
-        if (r == 0) {
-            fence_after();
-            issue(0, 0);
-            commit(bar);
+        if (tile_sync_or<I::kTileThreads>(tbar, !ok)) {
+            failed = true;
+            break;
         }
-        for (int l = 0; l <= kLayers; ++l) {
-            const bool ok = bar_wait(bar, phase);
+        stored(0);
+        // the next tile's queries; they are encoded while hidden layers' MMAs
+        // run (layer 0's, the only readers of the features, are done then)
+        const bool more = (tile + stride) * kRows < total;
+        if (more) load_raw(q + stride * kRows);
+        float y[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int l = 0; l < kLayers; ++l) {
+            if (l > 0 && more) encode_own(l - 1);
+            ok = bar_wait(bar, phase) && ok;
             phase ^= 1u;
-            if (wg_sync_or(wgbar, !ok)) {
-                failed = true;
-                break;
-            }
             fence_after();
-            const uint32_t acc = trow + (uint32_t)W * (uint32_t)(l % T::kAccBufs);
-            if (l == kLayers) {
-                float v[16];
-                tmem_ld16(acc, v);
+            // this thread's columns, 32 at a time
+#pragma unroll
+            for (int hb = 0; hb < W / I::kSplit / 32; ++hb) {
+                const uint32_t c0 = (uint32_t)(W / I::kSplit) * (uint32_t)part + 32u * (uint32_t)hb;
+                uint32_t v[32], h[16];
+                tmem_ld32(tmem + lanes + c0, v);
                 tmem_wait_ld();
-                y[0] = v[0];
-                y[1] = v[1];
-                y[2] = v[2];
-                break;
+#pragma unroll
+                for (int c = 0; c < 16; ++c)
+                    h[c] = pack2_relu(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1]));
+                tmem_st16(tmem_a + lanes + c0 / 2u, h);
             }
-            // tensor-memory loads per wait: four at width 128; one at width
-            // 64, whose two CTAs per SM leave 64 registers a thread
-            constexpr int kLd = W == 64 ? 1 : 4;
-#pragma unroll
-            for (int h = 0; h < (int)T::kKSubs; ++h) {  // 64-column K sub-tiles of H_{l+1}
-                unsigned char *At = A + (uint32_t)h * kSub;
-#pragma unroll
-                for (int c0 = 0; c0 < 4; c0 += kLd) {
-                    float v[kLd][16];
-#pragma unroll
-                    for (int c = 0; c < kLd; ++c) tmem_ld16(acc + 64 * h + 16 * (c0 + c), v[c]);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int c = 0; c < kLd; ++c) {
-                        uint4 lo, hi;
-                        lo.x = pack2_relu(v[c][0], v[c][1]);
-                        lo.y = pack2_relu(v[c][2], v[c][3]);
-                        lo.z = pack2_relu(v[c][4], v[c][5]);
-                        lo.w = pack2_relu(v[c][6], v[c][7]);
-                        hi.x = pack2_relu(v[c][8], v[c][9]);
-                        hi.y = pack2_relu(v[c][10], v[c][11]);
-                        hi.z = pack2_relu(v[c][12], v[c][13]);
-                        hi.w = pack2_relu(v[c][14], v[c][15]);
-                        *reinterpret_cast<uint4 *>(At + sw_off(r, 2 * (c0 + c))) = lo;
-                        *reinterpret_cast<uint4 *>(At + sw_off(r, 2 * (c0 + c) + 1)) = hi;
-                    }
-                }
-                // sub-tile h of H_{l+1} is written: layer l + 1's MMAs on it
-                // start while the next sub-tile is converted
-                fence_async_smem();
-                fence_before();
-                wg_sync(wgbar);
-                if (r == 0) {
-                    fence_after();
-                    issue(l + 1, h);
-                    if (h == (int)T::kKSubs - 1) commit(bar);
-                }
-            }
+            stored(l + 1);
         }
-        if (failed) break;
-        if (live) {
+        ok = bar_wait(bar, phase) && ok;
+        phase ^= 1u;
+        fence_after();
+        if (part == 0) {
+            float v[16];
+            tmem_ld16(tmem + lanes, v);
+            tmem_wait_ld();
+            y[0] = v[0];
+            y[1] = v[1];
+            y[2] = v[2];
+        }
+        if (live && ok && part == 0) {
             if (out) {
                 out[(size_t)q * 3 + 0] = y[0];
                 out[(size_t)q * 3 + 1] = y[1];
@@ -412,19 +510,18 @@ __global__ void __launch_bounds__(128 * tc::Tc<W>::kGroups) k_infer_tc(const uns
             }
         }
     }
+    failed = failed || !ok;
     if (failed) {
         // the MMAs of the timed-out phase may still be in flight: wait once
         // more (bounded) before the tensor memory is released
         bar_wait(bar, phase ^ 1u);
-        if (r == 0) atomicExch(err, 1);
+        atomicExch(err, 1);
     }
     fence_before();
     __syncthreads();
     if (warp == 0) {
         fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem - kGroupCols * (uint32_t)g),
-                     "r"(T::kInferTmemCols)
-                     : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(I::kCols) : "memory");
     }
 }
 
@@ -955,9 +1052,8 @@ void make_image(NrcState &N, cudaStream_t st) {
 template <int W>
 void launch_infer(NrcState &N, const float *raw, int stride, int n, const int *n_dev, float *out, float4 *rad,
                   cudaStream_t st) {
-    using T = tc::Tc<W>;
-    k_infer_tc<W><<<N.sms * T::kCtasPerSm, 128 * T::kGroups, T::kSmemBytes, st>>>(N.img, raw, stride, n, n_dev, out,
-                                                                                  rad, N.ints + 2);
+    using I = tc::Ti<W>;
+    k_infer_tc<W><<<N.sms, I::kTileThreads * I::kGroups, I::kSmemBytes, st>>>(N.img, raw, stride, n, n_dev, out, rad, N.ints + 2);
 }
 
 // cuTensorMapEncodeTiled, through the runtime's driver entry point.
@@ -1064,9 +1160,9 @@ kgk_status nrc_init(NrcState &N, const kgk_nrc_config *cfg, int device) {
     KGK_CUDA(cudaFuncSetAttribute(k_train_fb_tc<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)tc::Tc<128>::kSmemBytes));
     KGK_CUDA(cudaFuncSetAttribute(k_infer_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)tc::Tc<64>::kSmemBytes));
+                                  (int)tc::Ti<64>::kSmemBytes));
     KGK_CUDA(cudaFuncSetAttribute(k_infer_tc<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)tc::Tc<128>::kSmemBytes));
+                                  (int)tc::Ti<128>::kSmemBytes));
     cudaDeviceProp p;
     KGK_CUDA(cudaGetDeviceProperties(&p, device));
     N.sms = p.multiProcessorCount;
@@ -1097,8 +1193,7 @@ kgk_status nrc_check_error(NrcState &N) {
 
 kgk_status nrc_infer_dev(NrcState &N, const float *raw, int stride, int n, const int *n_dev, float *out, float4 *rad,
                          cudaStream_t st) {
-    // width 64: two ~107 KB CTAs of four warpgroups per SM (2 x 256 TMEM columns of 512);
-    // width 128: one ~213 KB CTA of two warpgroups per SM
+    // one CTA per SM (all of its tensor memory)
     if (N.cfg.width == 128) launch_infer<128>(N, raw, stride, n, n_dev, out, rad, st);
     else launch_infer<64>(N, raw, stride, n, n_dev, out, rad, st);
     KGK_CUDA(cudaGetLastError());
