@@ -53,3 +53,21 @@ def test_large_scene_leaves():
         info = s.build_bvh()
         s.validate_bvh()
     assert info["max_leaf_size"] == 1 and info["n_binary_nodes"] == 2 * 65537 - 1
+
+
+@pytest.mark.parametrize("n", [(1 << 20) - 1, (1 << 20) + 1])
+def test_large_level_chunks(n):
+    """The size of the chunks that large levels are binned and partitioned in
+    changes at 2^20 triangles."""
+    tris = soup(n, "random", n)
+    tris["verts"][:, 1:3, :3] = tris["verts"][:, :1, :3] + 0.02 * (tris["verts"][:, 1:3, :3] - tris["verts"][:, :1, :3])
+    rays = scenes.parity_rays(128, (-5, -5, -5), (5, 5, 5), seed=n)
+    with Scene(tris, np.stack([make_material()])) as s:
+        s.build_bvh()
+        s.validate_bvh()
+        ids, t = s.trace_closest(rays)
+    oids, ot = orc.closest_brute(tris, rays)
+    ok = orc.classify(tris, rays, oids, ot) == 0
+    assert np.array_equal(ids[ok], oids[ok])
+    hit = ok & (oids >= 0)
+    assert np.array_equal(t[hit], ot[hit])
