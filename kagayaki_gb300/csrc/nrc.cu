@@ -1212,8 +1212,11 @@ kgk_status nrc_grad_dev(NrcState &N, const float *raw, int raw_stride, const flo
         const size_t cnt = (size_t)(kLayers + 1) * rows * N.cfg.width;
         KGK_TRY(dalloc(&N.trH, cnt, "cache training scratch"));
         KGK_TRY(dalloc(&N.trD, cnt, "cache training scratch"));
-        KGK_CUDA(cudaMemset(N.trH, 0, cnt * sizeof(unsigned short)));
-        KGK_CUDA(cudaMemset(N.trD, 0, cnt * sizeof(unsigned short)));  // output-layer columns >= 8 stay 0
+        // Output-layer columns >= 8 stay 0; k_train_fb_tc writes all else that is
+        // read.  On the kernels' own stream: the scene's stream does not wait for
+        // the legacy one, and a late clear would wipe what they wrote.
+        const size_t layer = (size_t)rows * N.cfg.width;
+        KGK_CUDA(cudaMemsetAsync(N.trD + kLayers * layer, 0, layer * sizeof(unsigned short), st));
         N.tr_cap = rows;
     }
     KGK_CUDA(cudaMemsetAsync(N.g, 0, N.params * sizeof(float), st));

@@ -40,3 +40,25 @@ def test_prefixes(width):
         plain[[5, 9]] = 0.5
         ok[5] = False
         assert np.array_equal(infer(s, plain)[ok], full[ok])
+
+
+@pytest.mark.parametrize("width", [64, 128])
+def test_gradients_as_the_scratch_grows(width):
+    """Sizes around a tile and around one round of all tiles in flight, each
+    larger than the last, so that the call grows the training scratch; a second
+    call of the size finds it there.  The FP32 sums differ by their order only."""
+    tris, mats, _ = scenes.cornell_box()
+    rng = np.random.default_rng(width)
+    with Scene(tris, mats) as s:
+        s.cache_init(width=width, seed=3)
+        n_params = 64 * width + 4 * width * width + 3 * width
+        for n in (1, 127, 129, 4096, 152 * 2 * 128, 152 * 4 * 128 + 1, 1 << 17, 1 << 18):
+            raw = rng.random((n, 13), dtype=np.float32)
+            tgt = rng.random((n, 3), dtype=np.float32)
+            g = [np.full(n_params, np.nan, np.float32) for _ in range(2)]
+            for k in range(2):
+                check(lib().kgk_nrc_gradients(s._h, ctypes.c_void_p(raw.ctypes.data), ctypes.c_void_p(tgt.ctypes.data),
+                                              n, ctypes.c_void_p(g[k].ctypes.data), None))
+            norm = np.linalg.norm(g[1])
+            assert np.isfinite(norm) and norm > 0
+            assert np.linalg.norm(g[0] - g[1]) <= 1e-3 * norm, n
