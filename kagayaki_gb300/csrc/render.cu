@@ -1496,11 +1496,11 @@ template <class T> kgk_status ensure(T **p, size_t n, const char *what) {
     return dalloc(p, n, what);
 }
 
-kgk_status ensure_pixels(RenderState &R, int W, int H) {
+kgk_status ensure_pixels(RenderState &R, int W, int H, cudaStream_t st) {
     if (R.W == W && R.H == H && R.seeds) return KGK_OK;
     const size_t npx = (size_t)W * H;
     KGK_TRY(ensure(&R.seeds, npx, "per-pixel seeds"));
-    KGK_CUDA(cudaMemset(R.seeds, 0, npx * sizeof(unsigned long long)));
+    KGK_CUDA(cudaMemsetAsync(R.seeds, 0, npx * sizeof(unsigned long long), st));  // where the chain is read
     KGK_TRY(ensure(&R.frame, npx, "frame buffer"));
     KGK_TRY(ensure(&R.kept, npx, "frame buffer"));
     R.kept_valid = false;
@@ -1643,7 +1643,7 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
     // scene's stream (counter resets first) waits for them.
     if (R.shadowed) KGK_CUDA(cudaStreamWaitEvent(s->stream, R.shadowed, 0));
     const int W = cfg->width, H = cfg->height, npx = W * H;
-    KGK_TRY(ensure_pixels(R, W, H));
+    KGK_TRY(ensure_pixels(R, W, H, s->stream));
     if (cfg->estimator == KGK_ESTIMATOR_COMPAT && cfg->frame_index == 0)
         KGK_CUDA(cudaMemsetAsync(R.seeds, 0, (size_t)npx * sizeof(unsigned long long), s->stream));
     // samples per wave: compat chains the per-pixel seeds, one sample per wave

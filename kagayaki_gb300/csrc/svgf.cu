@@ -1418,7 +1418,7 @@ kgk_status kgk_svgf_output(kgk_scene *s, const kgk_svgf_config *cfg, const kgk_v
         KGK_TRY(dalloc(&S.col, npx, "SVGF colour"));
         KGK_TRY(dalloc(&S.tmp, npx, "SVGF colour"));
         KGK_TRY(dalloc(&S.compat_scratch, compat_scratch_bytes(npx), "SVGF scratch"));
-        KGK_CUDA(cudaMemset(S.prev, 0, npx * sizeof(kgk_svgf_buffer)));
+        KGK_CUDA(cudaMemsetAsync(S.prev, 0, npx * sizeof(kgk_svgf_buffer), s->stream));
         S.W = W;
         S.H = H;
         S.has_prev = false;
