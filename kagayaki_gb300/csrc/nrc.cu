@@ -51,7 +51,10 @@ __device__ __forceinline__ void sincospi_feature(float x, float *s, float *c) {
     __sincosf(r * 3.14159265358979f, s, c);
 }
 
-// Features 2 i and 2 i + 1 of a raw query, packed (see encode_row).
+// Features 2 i and 2 i + 1 of the 64 of a raw query, packed: 3 x 12 sine / cosine
+// features of the normalised position (6 octaves), normal and view direction,
+// their sines and cosines (12), roughness and albedo, six constant ones (the
+// biases).
 __device__ __forceinline__ uint32_t encode_pair(const float *raw, int i) {
     if (i < 18) {
         float s, co;
@@ -66,35 +69,6 @@ __device__ __forceinline__ uint32_t encode_pair(const float *raw, int i) {
     }
     if (i < 29) return pack2(raw[9 + 2 * (i - 27)], raw[10 + 2 * (i - 27)]);
     return pack2(1.0f, 1.0f);
-}
-
-// All 64 input features of a raw query: 3 x 12 sine / cosine features of the
-// normalised position (6 octaves), normal and view direction, their sines and
-// cosines (12), roughness and albedo, six constant ones (the biases).
-__device__ __forceinline__ void encode_row(const float *raw, float (&f)[64]) {
-#pragma unroll
-    for (int ax = 0; ax < 3; ++ax) {
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            float s, co;
-            sincospi_feature(raw[ax] * (float)(1 << k), &s, &co);
-            f[ax * 12 + 2 * k] = s;
-            f[ax * 12 + 2 * k + 1] = co;
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < 6; ++j) f[36 + j] = raw[3 + j];  // normal, view
-#pragma unroll
-    for (int j = 0; j < 6; ++j) {
-        float s, co;
-        sincospi_feature(raw[3 + j], &s, &co);
-        f[42 + 2 * j] = s;
-        f[42 + 2 * j + 1] = co;
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) f[54 + j] = raw[9 + j];  // roughness, albedo
-#pragma unroll
-    for (int j = 58; j < 64; ++j) f[j] = 1.0f;
 }
 
 // ---------------------------------------------------------------------------
@@ -235,20 +209,6 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 
 }  // namespace tc
 
-// Named barrier of one warpgroup (ids 1..4; 0 is __syncthreads), and its OR
-// reduction.
-__device__ __forceinline__ void wg_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
-__device__ __forceinline__ bool wg_sync_or(int id, bool v) {
-    uint32_t r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, %2, 128, p;\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}\n"
-        : "=r"(r)
-        : "r"((uint32_t)v), "r"(id)
-        : "memory");
-    return r != 0;
-}
-
 // Inference keeps the activations in tensor memory: a warpgroup's 128 x W
 // accumulator is read back, rounded and stored as the next layer's A operand
 // (W / 2 columns of BF16 pairs) beside it, and the MMA takes A from there.  In
@@ -316,7 +276,8 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 }  // namespace tc
 
-// Named barrier of the N threads of one tile, and its OR reduction.
+// Named barrier of the N threads of one tile (ids 1..4; 0 is __syncthreads), and
+// its OR reduction.
 template <int N>
 __device__ __forceinline__ void tile_sync(int id) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory");
@@ -528,8 +489,14 @@ __global__ void __launch_bounds__(tc::Ti<W>::kTileThreads * tc::Ti<W>::kGroups, 
 // ---------------------------------------------------------------------------
 // Training forward and backward on the 5th-generation tensor cores.  The CTA
 // layout is k_infer_tc's: the weights once in shared memory (K-major,
-// 128-byte swizzle), one 128-sample tile per warpgroup (thread r = row r =
-// tensor-memory lane r), a W-column FP32 accumulator per warpgroup.  Per tile:
+// 128-byte swizzle), one 128-sample tile per warpgroup, or per two at width
+// 128, each converting half of the columns (thread r = row r =
+// tensor-memory lane r), a W-column FP32 accumulator per tile.  2^18 samples at
+// width 128 take 200 us (210 with a warpgroup a tile) where the scratch alone
+// is 100 us of memory traffic; the rest is the chain of eleven dependent steps
+// of two tiles an SM, no part of which is most of it (without the stores 34 us
+// less, without waiting for them 20, with an eighth of the MMAs 22, without the
+// encoding 6).  Per tile:
 //   forward   Z_l = H_l W_l^T (A = H_l, B = W_l, both K-major), l = 0..4;
 //             H_{l+1} = bf16(relu(Z_l)), the ReLU derivative kept as bits;
 //             Y = H_5 W_5^T (N = 16, 3 live outputs);
@@ -548,20 +515,24 @@ __global__ void __launch_bounds__(tc::Ti<W>::kTileThreads * tc::Ti<W>::kGroups, 
 // freeing its tensor memory.
 // ---------------------------------------------------------------------------
 template <int W>
-__global__ void __launch_bounds__(128 * tc::Tc<W>::kGroups) k_train_fb_tc(
+__global__ void __launch_bounds__(tc::Ti<W>::kTileThreads * tc::Tc<W>::kGroups) k_train_fb_tc(
     const unsigned short *__restrict__ img, const float *__restrict__ raw, int raw_stride,
     const float *__restrict__ target, int tgt_stride, int n, const int *n_dev, const float *scale_p,
     unsigned short *Ds, size_t layer_stride, const __grid_constant__ CUtensorMap tmH,
     const __grid_constant__ CUtensorMap tmD, float *loss_sum, int *err) {
     using namespace tc;
     using T = Tc<W>;
-    constexpr int kG = T::kGroups, P = Net<W>::kPitch, kMW = W / 32;
+    constexpr int kG = T::kGroups, P = Net<W>::kPitch;
+    constexpr int kTile = Ti<W>::kTileThreads, kCols = W / Ti<W>::kSplit, kMW = kCols / 32;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;
     unsigned char *sm = smem_raw + pad;
     const uint32_t s0 = smem_u32(sm);
     const int tid = threadIdx.x, warp = tid >> 5;
-    const int g = tid >> 7, r = tid & 127;
+    const int g = tid / kTile, r = tid & 127;             // tile slot, row
+    const int part = (tid >> 7) % Ti<W>::kSplit;          // the kCols columns this thread converts
+    const int col0 = part * kCols;
+    const bool first = part == 0 && r == 0;               // issues the tile's MMAs and stores
     const int wgbar = 1 + g;
     constexpr int kChunks = W / 8;
     for (int i = tid; i < (kLayers * W + kOutRows) * kChunks; i += blockDim.x) {
@@ -577,7 +548,7 @@ __global__ void __launch_bounds__(128 * tc::Tc<W>::kGroups) k_train_fb_tc(
         *reinterpret_cast<uint4 *>(sm + dst) = *reinterpret_cast<const uint4 *>(img + (size_t)row * P + c * 8);
     }
     const uint32_t bar = s0 + T::kBarOff + 8u * (uint32_t)g;
-    if (r == 0) {
+    if (first) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -611,8 +582,8 @@ __global__ void __launch_bounds__(128 * tc::Tc<W>::kGroups) k_train_fb_tc(
     auto run_mma = [&](bool backward, int l, const CUtensorMap *map, int nsub, int q0) -> bool {
         fence_async_smem();
         fence_before();
-        wg_sync(wgbar);
-        if (r == 0) {
+        tile_sync<kTile>(wgbar);
+        if (first) {
             fence_after();
             const bool last = l == kLayers;
             const uint32_t boff = last ? T::kOutOff : T::layer_off(l);
@@ -646,8 +617,8 @@ __global__ void __launch_bounds__(128 * tc::Tc<W>::kGroups) k_train_fb_tc(
         }
         const bool ok = bar_wait(bar, phase);
         phase ^= 1u;
-        if (r == 0 && map) bulk_wait_read();  // the tile may be overwritten after the barrier below
-        if (wg_sync_or(wgbar, !ok)) return false;
+        if (first && map) bulk_wait_read();  // the tile may be overwritten after the barrier below
+        if (tile_sync_or<kTile>(wgbar, !ok)) return false;
         fence_after();
         return true;
     };
@@ -659,15 +630,15 @@ __global__ void __launch_bounds__(128 * tc::Tc<W>::kGroups) k_train_fb_tc(
             float rw[kRaw];
 #pragma unroll
             for (int k = 0; k < kRaw; ++k) rw[k] = live ? raw[(size_t)q * raw_stride + k] : 0.0f;
-            float f[64];
-            encode_row(rw, f);
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
+                // two warpgroups: quarters 0 and 3 / 1 and 2, much the same work
+                if (Ti<W>::kSplit > 1 && (part == 0) != (c < 2 || c >= 6)) continue;
                 uint4 v;
-                v.x = pack2(f[8 * c + 0], f[8 * c + 1]);
-                v.y = pack2(f[8 * c + 2], f[8 * c + 3]);
-                v.z = pack2(f[8 * c + 4], f[8 * c + 5]);
-                v.w = pack2(f[8 * c + 6], f[8 * c + 7]);
+                v.x = encode_pair(rw, 4 * c);
+                v.y = encode_pair(rw, 4 * c + 1);
+                v.z = encode_pair(rw, 4 * c + 2);
+                v.w = encode_pair(rw, 4 * c + 3);
                 *reinterpret_cast<uint4 *>(A + sw_off(r, c)) = v;
             }
         }
@@ -681,10 +652,10 @@ __global__ void __launch_bounds__(128 * tc::Tc<W>::kGroups) k_train_fb_tc(
             }
             if (l < kLayers) {
 #pragma unroll
-                for (int hb = 0; hb < W / 64; ++hb) {  // 64 columns per tensor-memory wait
+                for (int hb = 0; hb < kCols / 64; ++hb) {  // 64 columns per tensor-memory wait
                     float v[4][16];
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) tmem_ld16(trow + 64 * hb + 16 * c, v[c]);
+                    for (int c = 0; c < 4; ++c) tmem_ld16(trow + col0 + 64 * hb + 16 * c, v[c]);
                     tmem_wait_ld();
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
@@ -703,7 +674,7 @@ __global__ void __launch_bounds__(128 * tc::Tc<W>::kGroups) k_train_fb_tc(
                         hi.y = pack2_relu(v[c][10], v[c][11]);
                         hi.z = pack2_relu(v[c][12], v[c][13]);
                         hi.w = pack2_relu(v[c][14], v[c][15]);
-                        unsigned char *At = A + (uint32_t)hb * kSub;
+                        unsigned char *At = A + (uint32_t)(col0 / 64 + hb) * kSub;
                         *reinterpret_cast<uint4 *>(At + sw_off(r, (2 * cb) & 7)) = lo;
                         *reinterpret_cast<uint4 *>(At + sw_off(r, (2 * cb + 1) & 7)) = hi;
                     }
@@ -720,7 +691,7 @@ __global__ void __launch_bounds__(128 * tc::Tc<W>::kGroups) k_train_fb_tc(
         if (failed) break;
         // relative L2: d/dy (y - t)^2 / (y^2 + eps), denominator held constant
         float dy[3] = {0.0f, 0.0f, 0.0f};
-        if (live) {
+        if (live && part == 0) {
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const float tt = target[(size_t)q * tgt_stride + c];
@@ -730,7 +701,7 @@ __global__ void __launch_bounds__(128 * tc::Tc<W>::kGroups) k_train_fb_tc(
                 dy[c] = 2.0f * d / den * inv_n * S;
             }
         }
-        {
+        if (part == 0) {
             // dZ_5: 16 columns (chunks 0 and 1 of the first sub-tile), 3 live;
             // its scratch row by the thread (columns 0..7; 8.. stay zero)
             uint4 lo;
@@ -752,10 +723,10 @@ __global__ void __launch_bounds__(128 * tc::Tc<W>::kGroups) k_train_fb_tc(
             // backward MMA, or (dZ_0) straight to the scratch
             unsigned short *dout = drow + (size_t)(l - 1) * layer_stride;
 #pragma unroll
-            for (int hb = 0; hb < W / 64; ++hb) {
+            for (int hb = 0; hb < kCols / 64; ++hb) {
                 float v[4][16];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) tmem_ld16(trow + 64 * hb + 16 * c, v[c]);
+                for (int c = 0; c < 4; ++c) tmem_ld16(trow + col0 + 64 * hb + 16 * c, v[c]);
                 tmem_wait_ld();
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
@@ -774,12 +745,12 @@ __global__ void __launch_bounds__(128 * tc::Tc<W>::kGroups) k_train_fb_tc(
                     hi.z = pack2(v[c][12], v[c][13]);
                     hi.w = pack2(v[c][14], v[c][15]);
                     if (l > 1) {
-                        unsigned char *At = A + (uint32_t)hb * kSub;
+                        unsigned char *At = A + (uint32_t)(col0 / 64 + hb) * kSub;
                         *reinterpret_cast<uint4 *>(At + sw_off(r, (2 * cb) & 7)) = lo;
                         *reinterpret_cast<uint4 *>(At + sw_off(r, (2 * cb + 1) & 7)) = hi;
                     } else {
-                        *reinterpret_cast<uint4 *>(dout + 16 * cb) = lo;
-                        *reinterpret_cast<uint4 *>(dout + 16 * cb + 8) = hi;
+                        *reinterpret_cast<uint4 *>(dout + col0 + 16 * cb) = lo;
+                        *reinterpret_cast<uint4 *>(dout + col0 + 16 * cb + 8) = hi;
                     }
                 }
             }
@@ -788,9 +759,9 @@ __global__ void __launch_bounds__(128 * tc::Tc<W>::kGroups) k_train_fb_tc(
     }
     if (failed) {
         bar_wait(bar, phase ^ 1u);
-        if (r == 0) atomicExch(err, 1);
+        if (first) atomicExch(err, 1);
     }
-    if (r == 0) bulk_wait_all();
+    if (first) bulk_wait_all();
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(~0u, lsum, o);
     if ((tid & 31) == 0 && loss_sum) atomicAdd(loss_sum, lsum * inv_n);
@@ -1097,7 +1068,7 @@ kgk_status launch_grad(NrcState &N, const float *raw, int raw_stride, const floa
     KGK_TRY(scratch_map(&md, N.trD, W, N.tr_cap));
     // as many CTAs as the batch's 128-row tiles need (one per warpgroup), at most the resident count
     const int fb_ctas = std::max(1, std::min(N.sms * T::kCtasPerSm, ((n + 127) / 128 + T::kGroups - 1) / T::kGroups));
-    k_train_fb_tc<W><<<fb_ctas, 128 * T::kGroups, T::kSmemBytes, st>>>(
+    k_train_fb_tc<W><<<fb_ctas, tc::Ti<W>::kTileThreads * T::kGroups, T::kSmemBytes, st>>>(
         N.img, raw, raw_stride, tgt, tgt_stride, n, n_dev, N.scal, N.trD, ls, mh, md, N.scal + 1, N.ints + 2);
     // split K: chunks of whole 64-row boxes, about two CTAs per SM over the six layers
     const int want = std::max(1, 2 * N.sms / (kLayers + 1));
