@@ -51,8 +51,7 @@ constexpr int kSmall = 2048;   // tasks up to this size build inside one block
 // each, so its quantised child box culls that triangle alone, and a node
 // yields at most 8 triangle tests.  Measured on the C2 frame (5.2M
 // triangles): 3089 Mrays/s at 1, 2978 at 2, 2799 at 3 (extend 43.5 / 46.0 /
-// 50.3 ms), for 1.72M / 1.00M / 0.71M wide nodes and a 140 / 87 / 65 ms
-// build.  Three for small scenes, whose nodes and triangles stay in cache:
+// 50.3 ms), for 1.72M / 1.00M / 0.71M wide nodes.  Three for small scenes, whose nodes and triangles stay in cache:
 // the 36-triangle Cornell box (C1) runs 1509 Mrays/s at 3, 1156 at 1.
 constexpr int kMaxLeaf = 3;                // the largest leaf the node format holds (8 x 3 = 24 bits)
 constexpr int kLeafLarge = 1;
@@ -552,13 +551,31 @@ __device__ WarpSplit sb_best_split(const int *bins, int *n_left) {
     return best;
 }
 
+// Inclusive minimum / maximum over a lane's segment [sb, ..], up to its lane; the
+// longest segment of the warp has `longest` lanes.
+__device__ __forceinline__ void seg_scan_box(float3 &lo, float3 &hi, int sb, int longest) {
+    const int lane = threadIdx.x & 31;
+    for (int o = 1; o < longest; o <<= 1) {
+        const float3 l = shfl_up3(lo, o), h = shfl_up3(hi, o);
+        if (lane - o >= sb) {
+            lo = fmin3(lo, l);
+            hi = fmax3(hi, h);
+        }
+    }
+}
+
 // Finishes the subtree of at most 32 primitives at refs [b, b + c) of the
 // task: lane i holds primitive i, the nodes of one level are segments of
 // lanes, and all of them are split at once.  A segment's candidate planes are
 // its primitives' own bins (an empty bin's plane makes the same partition as
-// the occupied bin before it, at a larger index), so lane i sums the boxes
-// left and right of its bin on each axis by walking its segment; the choice
-// (least cost, then lowest axis, then lowest bin) is that of the 32-bin scan.
+// the occupied bin before it, at a larger index).  The lanes take their segment
+// in the order of an axis's bins (ranks counted for the three axes at once, a
+// byte each) and the boxes left and right of every plane are scans from both
+// ends; the choice (least cost, then lowest axis, then lowest bin) is that of
+// the 32-bin scan.  Instruction issue bounds the small builder, most of it here;
+// with every lane walking its segment for the sums instead of scans, 5.2M
+// triangles took 3.48 for 3.10 ms in it (walking only segments of up to 4
+// or 8 lanes: no difference).
 __device__ void tiny_build(SbShared &sh, int root, int b, int c, int begin, int slot_base, int max_leaf,
                            BinNode *nodes, int *bfirst, int *bcount) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -576,59 +593,59 @@ __device__ void tiny_build(SbShared &sh, int root, int b, int c, int begin, int 
         if (longest == 0) break;
         const float3 cen = f3(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z));
         float3 clo = cen, chi = cen;
-        for (int k = 0; k < longest; ++k) {
-            const float3 q = shfl3(cen, min(sb + k, se - 1));
-            clo = fmin3(clo, q);
-            chi = fmax3(chi, q);
-        }
+        seg_scan_box(clo, chi, sb, longest);
+        clo = shfl3(clo, se - 1);
+        chi = shfl3(chi, se - 1);
         unsigned bin[3];
 #pragma unroll
         for (int a = 0; a < 3; ++a)
             bin[a] = (unsigned)bin_of(comp(cen, a), comp(clo, a), bin_scale(comp(clo, a), comp(chi, a)));
         const unsigned packed = bin[0] | bin[1] << 8 | bin[2] << 16;
-        float3 llo[3], lhi[3], rlo[3], rhi[3];
-        int lc[3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            llo[a] = rlo[a] = f3(INFINITY, INFINITY, INFINITY);
-            lhi[a] = rhi[a] = f3(-INFINITY, -INFINITY, -INFINITY);
-            lc[a] = 0;
-        }
-        for (int k = 0; k < longest; ++k) {
-            // past the segment's end the last primitive again: boxes do not change, counts skip it
-            const int src = min(sb + k, se - 1), in = sb + k < se ? 1 : 0;
-            const float3 ql = shfl3(lo, src), qh = shfl3(hi, src);
-            const unsigned qb = __shfl_sync(~0u, packed, src);
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                if (((qb >> (8 * a)) & 0xffu) <= bin[a]) {
-                    llo[a] = fmin3(llo[a], ql);
-                    lhi[a] = fmax3(lhi[a], qh);
-                    lc[a] += in;
-                } else {
-                    rlo[a] = fmin3(rlo[a], ql);
-                    rhi[a] = fmax3(rhi[a], qh);
-                }
-            }
-        }
         float cost = INFINITY;
         int key = 0x7fffffff;  // axis, bin
+        // each lane's rank in its segment by (bin, lane), per axis: a byte of
+        // d has its top bit set where the other's bin, or in a tie its lane,
+        // is the lower one
+        const unsigned mine2 = 2u * packed, base = 0x7f7f7fu + mine2;
+        unsigned rank = 0u;
+        for (int k = 0; k < longest; ++k) {
+            const int src = sb + k;
+            const unsigned other = __shfl_sync(~0u, mine2, src);
+            const unsigned d = base + (src < lane ? 0x010101u : 0u) - other;
+            if (k < s) rank += (d >> 7) & 0x010101u;
+        }
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            const int rc = s - lc[a];
-            if (rc > 0) {
-                const float ca = surface_area(llo[a], lhi[a]) * (float)lc[a] + surface_area(rlo[a], rhi[a]) * (float)rc;
-                if (ca < cost) { cost = ca; key = a * kBins + (int)bin[a]; }
+            sh.perm[warp][sb + ((rank >> (8 * a)) & 0xffu)] = (unsigned char)lane;
+            __syncwarp();
+            const int src = sh.perm[warp][lane];
+            __syncwarp();
+            float3 llo = shfl3(lo, src), lhi = shfl3(hi, src), rlo = llo, rhi = lhi;
+            const unsigned b = (__shfl_sync(~0u, packed, src) >> (8 * a)) & 0xffu;
+            for (int o = 1; o < longest; o <<= 1) {
+                const float3 ul = shfl_up3(llo, o), uh = shfl_up3(lhi, o);
+                const float3 dl = shfl_down3(rlo, o), dh = shfl_down3(rhi, o);
+                if (lane - o >= sb) { llo = fmin3(llo, ul); lhi = fmax3(lhi, uh); }
+                if (lane + o < se) { rlo = fmin3(rlo, dl); rhi = fmax3(rhi, dh); }
+            }
+            rlo = shfl_down3(rlo, 1);
+            rhi = shfl_down3(rhi, 1);
+            const unsigned nb = __shfl_down_sync(~0u, b, 1);
+            if (lane + 1 < se && nb != b) {  // the last primitive of its bin: a plane
+                const int lc = lane - sb + 1, rc = se - lane - 1;
+                const float ca = surface_area(llo, lhi) * (float)lc + surface_area(rlo, rhi) * (float)rc;
+                if (ca < cost) { cost = ca; key = a * kBins + (int)b; }
             }
         }
         float best = cost;
         int bkey = key;
-        for (int k = 0; k < longest; ++k) {
-            const int src = min(sb + k, se - 1);
-            const float q = __shfl_sync(~0u, cost, src);
-            const int qk = __shfl_sync(~0u, key, src);
-            if (q < best || (q == best && qk < bkey)) { best = q; bkey = qk; }
+        for (int o = 1; o < longest; o <<= 1) {
+            const float q = __shfl_up_sync(~0u, best, o);
+            const int qk = __shfl_up_sync(~0u, bkey, o);
+            if (lane - o >= sb && (q < best || (q == best && qk < bkey))) { best = q; bkey = qk; }
         }
+        best = __shfl_sync(~0u, best, se - 1);
+        bkey = __shfl_sync(~0u, bkey, se - 1);
         // no plane (all centroids in one bin on every axis): by position
         bool left = lane - sb < s / 2;
         if (best < INFINITY) {
@@ -660,13 +677,8 @@ __device__ void tiny_build(SbShared &sh, int root, int b, int c, int begin, int 
             se = right ? se : mid;
         }
         float3 nlo = lo, nhi = hi;
-        const int longest2 = __reduce_max_sync(~0u, act ? se - sb : 0);
-        for (int k = 0; k < longest2; ++k) {
-            const int q = min(sb + k, se - 1);
-            nlo = fmin3(nlo, shfl3(lo, q));
-            nhi = fmax3(nhi, shfl3(hi, q));
-        }
-        if (act && lane == sb)
+        seg_scan_box(nlo, nhi, sb, __reduce_max_sync(~0u, act ? se - sb : 0));
+        if (act && lane == se - 1)
             put_node(nodes, bfirst, bcount, node, nlo, nhi, begin + b + sb, se - sb, se - sb <= max_leaf);
     }
     if (mine) sh.idx[b + lane] = (unsigned short)local;
