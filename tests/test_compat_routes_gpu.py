@@ -6,7 +6,7 @@ pixel limit."""
 import numpy as np
 import pytest
 
-from kagayaki_gb300 import ESTIMATOR_COMPAT, Scene, camera_setup, scenes
+from kagayaki_gb300 import ESTIMATOR_COMPAT, ESTIMATOR_UNBIASED, Scene, camera_setup, scenes
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +44,20 @@ def test_routes_agree(kind, W, H, spp, depth):
     assert np.array_equal(ma, mb, equal_nan=True) and np.array_equal(va, vb, equal_nan=True)
     for k in ("Albedo", "Normal", "Depth", "MaterialID", "ObjectID"):
         assert np.array_equal(ra[k], rb[k], equal_nan=ra[k].dtype.kind == "f"), k
+
+
+@pytest.mark.parametrize("kind", ["cornell", "disney"])
+@pytest.mark.parametrize("W,H,spp", [(1, 1, 1), (97, 61, 3), (640, 300, 1), (333, 207, 4)])
+def test_small_tree_loops_agree(kind, W, H, spp):
+    """Waves on a small scene trace a ray per lane, on a larger one by the warp's
+    (ray, triangle) pairs: the same hits, so the same unbiased frames."""
+    tris, mats, c, tex, env = scenes.parity_scene(kind)
+    got = []
+    for t in (tris, far_away(tris, 2000)):
+        with Scene(t, mats, textures=tex, env=env) as s:
+            s.build_bvh()
+            cam = camera_setup(c["origin"], c["dist"], c["rot"], H)
+            img, st = s.render(cam, W, H, spp=spp, estimator=ESTIMATOR_UNBIASED)
+            got.append((img, (st["rays_closest"], st["rays_shadow"], st["paths"])))
+    assert np.array_equal(got[0][0], got[1][0], equal_nan=True)
+    assert got[0][1] == got[1][1]
