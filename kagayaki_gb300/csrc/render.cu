@@ -1892,10 +1892,15 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
     // reference's estimator at 640 x 480 x 4 / the unbiased at 1080p x 8, ms:
     // 642 triangles 1.38 : 1.38 / 3.6 : 3.85, 1,282 1.41 : 1.42 / 3.98 : 4.14,
     // 2,562 1.59 : 1.54 / 3.68 : 3.85 and 1.44 : 1.42 / 5.1 : 5.0.
+    // Blocks of large waves finish at different times; three times what fits at
+    // once evens them out (1080p, reference's estimator, a sample a wave: 1.27 ->
+    // 1.245 ms on the box; unbiased, 8 samples: 8.03 -> 7.79 ms), but costs small
+    // waves (640 x 480: 1.56 -> 1.61 ms).
     const bool loops = s->dev.n_tris <= kLoopTris;
+    const int loop_grid = (size_t)npx * std::min(spw, (int)cfg->spp) >= (1u << 20) ? 3 * grid : grid;
     auto shadow = [&](int q) {
         const int ci = q ? kSH1 : kSH0, fi = q ? kFS1 : kFS0;
-        if (loops) k_shadow_loop<<<grid, 128, 0, sh_st>>>(P, ci, R.sh_o[q], R.sh_d[q], R.sh_c[q]);
+        if (loops) k_shadow_loop<<<loop_grid, 128, 0, sh_st>>>(P, ci, R.sh_o[q], R.sh_d[q], R.sh_c[q]);
         else k_shadow<<<grid, 128, 0, sh_st>>>(P, ci, fi, R.sh_o[q], R.sh_d[q], R.sh_c[q]);
     };
     for (int done = by_pixel ? cfg->spp : 0, wave = 0; done < cfg->spp; done += spw, ++wave) {
@@ -1951,9 +1956,9 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
             KGK_CUDA(cudaMemsetAsync(R.cnt + nidx, 0, sizeof(int), st));
             KGK_TRY(stage_begin(0));
             if (cfg->count_work)
-                (loops ? k_extend_loop<true> : k_extend<true>)<<<grid, 128, 0, st>>>(P, cidx, n, R.mq, R.lq, R.dq);
+                (loops ? k_extend_loop<true> : k_extend<true>)<<<loops ? loop_grid : grid, 128, 0, st>>>(P, cidx, n, R.mq, R.lq, R.dq);
             else
-                (loops ? k_extend_loop<false> : k_extend<false>)<<<grid, 128, 0, st>>>(P, cidx, n, R.mq, R.lq, R.dq);
+                (loops ? k_extend_loop<false> : k_extend<false>)<<<loops ? loop_grid : grid, 128, 0, st>>>(P, cidx, n, R.mq, R.lq, R.dq);
             KGK_TRY(stage_end());
             ++extend_launches;
             // shading adds to the radiance the previous shadow passes wrote and
