@@ -490,7 +490,10 @@ typedef struct kgk_nrc_config {
     int32_t train_steps;        /* Adam steps per frame, 4                       */
     float spread_c;             /* termination: path spread^2 > c * footprint^2  */
     uint64_t seed;              /* weight initialisation                          */
-    int32_t reserved[8];
+    int32_t give_up_waits;      /* 1: the kernels' waits for their tensor-core work give up
+                                 * at once, as they do after about a second: every call
+                                 * that runs them returns KGK_ERR_DEVICE_CHECK (tests)   */
+    int32_t reserved[7];
 } kgk_nrc_config;
 
 /* (Re)initialises the scene's cache with He-uniform weights. */

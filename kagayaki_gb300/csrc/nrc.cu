@@ -85,8 +85,9 @@ __device__ __forceinline__ uint32_t encode_pair(const float *raw, int i) {
 // (k_train_fb_tc) in shared memory, from where they also go to its scratch.
 // Tiles synchronise on their own named barriers, so the CUDA-core work of one
 // overlaps the MMAs of another.  The output layer uses N=16 (3 live rows of the
-// padded weights).  Every wait is bounded: on a timeout the CTA raises *err,
-// stops issuing and frees its tensor memory.
+// padded weights).  Every wait is bounded: on a timeout the tile raises *err and
+// issues no more, and the CTA frees its tensor memory after one more (bounded)
+// wait for what is in flight.
 // ---------------------------------------------------------------------------
 namespace tc {
 
@@ -294,7 +295,10 @@ __device__ __forceinline__ bool tile_sync_or(int id, bool v) {
     return r != 0;
 }
 
-template <int W>
+// kGiveUp: every wait before the last one runs out at once (an instance of its
+// own, for tests of that path: a limit handed in at run time costs 2 %; what the
+// waits' outcome itself costs, the vote and the branches on it, is 0.8 %).
+template <int W, bool kGiveUp>
 __global__ void __launch_bounds__(tc::Ti<W>::kTileThreads * tc::Ti<W>::kGroups, 1)
     k_infer_tc(const unsigned short *__restrict__ img, const float *__restrict__ raw, int stride_floats, int n,
                const int *n_dev, float *out, float4 *rad, int *err) {
@@ -346,7 +350,7 @@ __global__ void __launch_bounds__(tc::Ti<W>::kTileThreads * tc::Ti<W>::kGroups, 
     const uint32_t tmem_f = tmem_a + (uint32_t)W / 2;                  // features: A operand of layer 0
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;          // this warp's 32 lanes
     const int total = n_dev ? min(*n_dev, n) : n;
-    uint32_t phase = 0;
+    uint32_t phase = 0, issued = 1;  // parities: the next wait's, the last commit's
     bool failed = false, ok = true;
     const uint64_t bdesc = sw128_desc(s0);  // + offsets in 16 B units
     // the MMAs of layer l, issued once every row's A is stored
@@ -365,18 +369,29 @@ __global__ void __launch_bounds__(tc::Ti<W>::kTileThreads * tc::Ti<W>::kGroups, 
                         kk > 0 ? 1u : 0u);
         }
         commit(bar);
+        issued ^= 1u;
     };
-    // A is stored (by every row: the barrier) -> layer l's MMAs
+    // A is stored (by every row: the barrier) -> layer l's MMAs, unless those
+    // before may still be in flight: the issuing thread's own waits say so, and
+    // nobody else's need to be asked for
     auto stored = [&](int l) {
         if (l > 0) {  // layer 0's barrier is the tile's own, below
             tmem_wait_st();
             fence_before();
             tile_sync<I::kTileThreads>(tbar);
         }
-        if (first) {
+        if (first && ok) {
             fence_after();
             issue(l);
         }
+    };
+    // Waits for the MMAs issued last; ok: they and all before are done, for
+    // every lane of the warp, which reads and writes tensor memory together.  A
+    // warp whose wait ran out leaves tensor memory alone.
+    auto wait_mma = [&]() {
+        ok = __all_sync(~0u, !kGiveUp && bar_wait(bar, phase)) && ok;
+        phase ^= 1u;
+        fence_after();
     };
     float rw[kRaw];
     auto load_raw = [&](int q) {
@@ -408,8 +423,7 @@ __global__ void __launch_bounds__(tc::Ti<W>::kTileThreads * tc::Ti<W>::kGroups, 
         const int q = tile * kRows + r;
         const bool live = q < total;
         // the barrier before layer 0 tells all of the tile's threads whether a
-        // wait timed out in any of them (inside a tile they go on: every wait
-        // is bounded)
+        // wait ran out in any of them (inside a tile they go on)
         tmem_wait_st();
         fence_before();
         if (tile_sync_or<I::kTileThreads>(tbar, !ok)) {
@@ -424,28 +438,26 @@ __global__ void __launch_bounds__(tc::Ti<W>::kTileThreads * tc::Ti<W>::kGroups, 
         float y[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
         for (int l = 0; l < kLayers; ++l) {
-            if (l > 0 && more) encode_own(l - 1);
-            ok = bar_wait(bar, phase) && ok;
-            phase ^= 1u;
-            fence_after();
-            // this thread's columns, 32 at a time
+            if (l > 0 && more && ok) encode_own(l - 1);
+            wait_mma();
+            if (ok) {
+                // this thread's columns, 32 at a time
 #pragma unroll
-            for (int hb = 0; hb < W / I::kSplit / 32; ++hb) {
-                const uint32_t c0 = (uint32_t)(W / I::kSplit) * (uint32_t)part + 32u * (uint32_t)hb;
-                uint32_t v[32], h[16];
-                tmem_ld32(tmem + lanes + c0, v);
-                tmem_wait_ld();
+                for (int hb = 0; hb < W / I::kSplit / 32; ++hb) {
+                    const uint32_t c0 = (uint32_t)(W / I::kSplit) * (uint32_t)part + 32u * (uint32_t)hb;
+                    uint32_t v[32], h[16];
+                    tmem_ld32(tmem + lanes + c0, v);
+                    tmem_wait_ld();
 #pragma unroll
-                for (int c = 0; c < 16; ++c)
-                    h[c] = pack2_relu(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1]));
-                tmem_st16(tmem_a + lanes + c0 / 2u, h);
+                    for (int c = 0; c < 16; ++c)
+                        h[c] = pack2_relu(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1]));
+                    tmem_st16(tmem_a + lanes + c0 / 2u, h);
+                }
             }
             stored(l + 1);
         }
-        ok = bar_wait(bar, phase) && ok;
-        phase ^= 1u;
-        fence_after();
-        if (part == 0) {
+        wait_mma();
+        if (part == 0 && ok) {
             float v[16];
             tmem_ld16(tmem + lanes, v);
             tmem_wait_ld();
@@ -473,9 +485,9 @@ __global__ void __launch_bounds__(tc::Ti<W>::kTileThreads * tc::Ti<W>::kGroups, 
     }
     failed = failed || !ok;
     if (failed) {
-        // the MMAs of the timed-out phase may still be in flight: wait once
-        // more (bounded) before the tensor memory is released
-        bar_wait(bar, phase ^ 1u);
+        // the MMAs committed last may still be in flight: the thread that issued
+        // them waits once more (bounded) before the tensor memory is released
+        if (first) bar_wait(bar, issued);
         atomicExch(err, 1);
     }
     fence_before();
@@ -1024,7 +1036,8 @@ template <int W>
 void launch_infer(NrcState &N, const float *raw, int stride, int n, const int *n_dev, float *out, float4 *rad,
                   cudaStream_t st) {
     using I = tc::Ti<W>;
-    k_infer_tc<W><<<N.sms, I::kTileThreads * I::kGroups, I::kSmemBytes, st>>>(N.img, raw, stride, n, n_dev, out, rad, N.ints + 2);
+    auto *k = N.cfg.give_up_waits ? k_infer_tc<W, true> : k_infer_tc<W, false>;
+    k<<<N.sms, I::kTileThreads * I::kGroups, I::kSmemBytes, st>>>(N.img, raw, stride, n, n_dev, out, rad, N.ints + 2);
 }
 
 // cuTensorMapEncodeTiled, through the runtime's driver entry point.
@@ -1130,10 +1143,16 @@ kgk_status nrc_init(NrcState &N, const kgk_nrc_config *cfg, int device) {
                                   (int)tc::Tc<64>::kSmemBytes));
     KGK_CUDA(cudaFuncSetAttribute(k_train_fb_tc<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)tc::Tc<128>::kSmemBytes));
-    KGK_CUDA(cudaFuncSetAttribute(k_infer_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    KGK_CUDA(cudaFuncSetAttribute(k_infer_tc<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)tc::Ti<64>::kSmemBytes));
-    KGK_CUDA(cudaFuncSetAttribute(k_infer_tc<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    KGK_CUDA(cudaFuncSetAttribute(k_infer_tc<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)tc::Ti<128>::kSmemBytes));
+    if (N.cfg.give_up_waits) {
+        KGK_CUDA(cudaFuncSetAttribute(k_infer_tc<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)tc::Ti<64>::kSmemBytes));
+        KGK_CUDA(cudaFuncSetAttribute(k_infer_tc<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)tc::Ti<128>::kSmemBytes));
+    }
     cudaDeviceProp p;
     KGK_CUDA(cudaGetDeviceProperties(&p, device));
     N.sms = p.multiProcessorCount;

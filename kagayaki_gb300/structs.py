@@ -131,7 +131,7 @@ class KgkNrcConfig(ctypes.Structure):
                 ("learning_rate", ctypes.c_float), ("train_paths", ctypes.c_int32),
                 ("train_suffix_max", ctypes.c_int32), ("train_steps", ctypes.c_int32),
                 ("spread_c", ctypes.c_float), ("seed", ctypes.c_uint64),
-                ("reserved", ctypes.c_int32 * 8)]
+                ("give_up_waits", ctypes.c_int32), ("reserved", ctypes.c_int32 * 7)]
 
 
 assert ctypes.sizeof(KgkCamera) == 72
