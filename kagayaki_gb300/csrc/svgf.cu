@@ -107,6 +107,14 @@ struct CompatArgs {
     kgk_vec *hist;
 };
 
+// The pixel that c was in the frame before; -1 without one, also where the
+// position it names lies outside the image (records are the caller's).
+__device__ __forceinline__ int prev_pixel(const CompatArgs &a, const kgk_svgf_buffer &c) {
+    if (a.frame == 0 || c.PosLastFrameI[0] == -1) return -1;
+    const long long p = (long long)a.W * c.PosLastFrameI[1] + c.PosLastFrameI[0];
+    return p < 0 || p >= (long long)a.W * a.H ? -1 : (int)p;
+}
+
 #define FOR_PIXELS(n) for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < (n); p += gridDim.x * blockDim.x)
 
 // save_png's tone mapping on the device.  tone_host's bytes are a step
@@ -207,21 +215,17 @@ __global__ void k_c_front(CompatArgs a) {
         if (store) a.R[p] = kv(r);
         const float l = lumf(div3(r, v3(c.Albedo) + f3(kS, kS, kS)));
         float m1 = l, m2 = l * l;
-        bool sp = a.frame == 0 || px == -1;
+        const int prev = prev_pixel(a, c);
+        const bool sp = prev < 0 || a.P[prev].sampleNum < 3;
         if (!sp) {
-            const int prev = W * py + px;
-            if (prev < 0 || prev >= W * H || a.P[prev].sampleNum < 3) {
-                sp = true;
-            } else {
-                const int n = a.P[prev].sampleNum + 1;
-                float cw = 1.0f / 5.0f;
-                if (n < 5) cw = 1.0f / (float)n;
-                m1 = (1.0f - cw) * a.P[prev].MomentOne + cw * m1;
-                m2 = (1.0f - cw) * a.P[prev].MomentTwo + cw * m2;
-                c.sampleNum = n;
-                c.MomentOne = m1;
-                c.MomentTwo = m2;
-            }
+            const int n = a.P[prev].sampleNum + 1;
+            float cw = 1.0f / 5.0f;
+            if (n < 5) cw = 1.0f / (float)n;
+            m1 = (1.0f - cw) * a.P[prev].MomentOne + cw * m1;
+            m2 = (1.0f - cw) * a.P[prev].MomentTwo + cw * m2;
+            c.sampleNum = n;
+            c.MomentOne = m1;
+            c.MomentTwo = m2;
         }
         a.M1[p] = m1;
         a.M2[p] = m2;
@@ -324,8 +328,8 @@ __global__ void __launch_bounds__(256) k_c_var(CompatArgs a) {
     if (sp) {
         r.MomentOne = m1;
         r.MomentTwo = m2;
-        if (a.frame == 0 || r.PosLastFrameI[0] == -1) r.sampleNum = 1;
-        else r.sampleNum = a.P[W * r.PosLastFrameI[1] + r.PosLastFrameI[0]].sampleNum + 1;
+        const int prev = prev_pixel(a, r);
+        r.sampleNum = prev < 0 ? 1 : a.P[prev].sampleNum + 1;
     }
     a.mv2[p] = make_int2(own.y, __float_as_int(fminf(fmaxf(0.0f, m2 - m1 * m1), 1000.0f)));
 }
