@@ -71,10 +71,14 @@ constexpr float kLog2e = 1.44269504088896341f;
 // exp(-|d - nd| / (|dx gx + dy gy| + sINF)) and the luminance weight
 // exp(-|l - nl| / (4 sd + sINF)) share one base-2 exponential of the sum of
 // their arguments, each a product with a reciprocal (the luminance one taken
-// once per pixel): an argument x carries a relative 2^-22 and so does the
-// exponential, below the 128 u of the normal weight's seven squarings.
+// once per pixel).  An argument x carries a relative 2^-21, so the weight 2^x a
+// relative |x| ln 2 2^-21 and the exponential's 2^-22: most where the weight is
+// least (x = -100: 2^-15 of 2^-100), and never more than 2^-21 in absolute terms,
+// as 2^x |x| ln 2 is at most 1 / e.
+// The quotient is formed with both sides a quarter: __fdividef gives 0 for a
+// divisor above 2^126, which slopes of 10^38 reach.
 __device__ __forceinline__ float depth_arg(float d, float nd, float slope) {
-    return __fdividef(-kLog2e * fabsf(d - nd), fabsf(slope) + kS);
+    return __fdividef(-0.25f * kLog2e * fabsf(d - nd), fmaf(0.25f, fabsf(slope), 0.25f * kS));
 }
 __device__ __forceinline__ float normal_w(float3 n, float3 m) {
     float c = fmaxf(0.0f, dot3(n, m));
