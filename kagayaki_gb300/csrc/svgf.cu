@@ -425,7 +425,7 @@ struct CompatPx {
     int2 om;          // own material and variance
     float3 n;
     float d, l, gx, gy;
-    float rl;         // the luminance weight's factor of |l - nl| (0: no luminance weight)
+    float rl;         // the luminance weight's factor of |l - nl|
     float bright;     // a tap brighter than this is left out
     float3 srad;
     float svar, swt;
@@ -442,7 +442,7 @@ struct CompatPx {
         const float2 g = reinterpret_cast<const float2 *>(a.gz)[p];
         gx = g.x;
         gy = g.y;
-        rl = af.w != 0.0f ? __fdividef(-kLog2e, 4.0f * a.sd[p] + kS) : 0.0f;
+        rl = __fdividef(-kLog2e, 4.0f * a.sd[p] + kS);
         // SVGF.cuh:405-411, whose first two bounds compare in double
         bright = (double)l > 0.5 ? 5 * l : (double)l > 0.1 ? 50 * l : l > kS ? 100 * l : INFINITY;
         srad = f3(0.0f, 0.0f, 0.0f);
@@ -456,9 +456,12 @@ struct CompatPx {
     // a neighbour at (qx, qy); absolute coordinates in the depth weight, SVGF.cuh:426
     __device__ __forceinline__ void tap(float h, int qx, int qy, int2 eo, float4 em, float4 eg) {
         if (eo.y < 0 || em.w > bright) return;
-        const float e = depth_arg(d, eg.w, (float)qx * gx + (float)qy * gy) + fminf(fabsf(l - em.w), 3e38f) * rl;
-        float w = h * ex2a(e) * normal_w(n, f3(eg));
-        w = om.x == eo.x ? w : 0.0f;
+        // where a value is not a number the weight is none either: the luminance
+        // term is left out, not multiplied by 0, where the pixel has none, and
+        // another material's weight is multiplied by 0
+        float e = depth_arg(d, eg.w, (float)qx * gx + (float)qy * gy);
+        if (af.w != 0.0f) e = fmaf(fabsf(l - em.w), rl, e);
+        const float w = (om.x == eo.x ? h : 0.0f) * ex2a(e) * normal_w(n, f3(eg));
         srad += f3(em) * w;
         svar += w * w * __int_as_float(eo.y);
         swt += w;
