@@ -39,9 +39,9 @@ struct NrcState {
     unsigned short *trH = nullptr;   // training scratch: activations H_l, [layer][row][width]
     unsigned short *trD = nullptr;   // training scratch: output gradients dZ_l, [layer][row][width]
     int tr_cap = 0;                  // rows the scratch holds
-    float *scal = nullptr;           // [0] loss scale, [1] last loss
-    int *ints = nullptr;             // [0] non-finite flag, [1] clean steps since the last scale change,
-                                     // [2] inference timeout flag
+    float *scal = nullptr;           // [0] loss scale, [1] last loss; the ints follow
+    int *ints = nullptr;             // scal + 4: [0] non-finite flag, [1] clean steps since the last scale
+                                     // change, [2] a kernel gave up a wait
     int step = 0;
     int sms = 0;
     int params = 0;                  // master weights (20,672 at width 64, 74,112 at 128)
@@ -55,13 +55,14 @@ void nrc_free(NrcState &N);
 // floats 13..15 and the path id (int bits) at float 16 of each record.
 kgk_status nrc_infer_dev(NrcState &N, const float *raw, int stride, int n, const int *n_dev, float *out, float4 *rad,
                          cudaStream_t st);
-// KGK_ERR_DEVICE_CHECK (and clears the flag) when an inference kernel gave up
-// a bounded wait; synchronous.
-kgk_status nrc_check_error(NrcState &N);
+// Waits for the stream.  KGK_ERR_DEVICE_CHECK (and clears the flag) when a kernel
+// gave up a bounded wait; else *loss (may be null) is the last loss.
+kgk_status nrc_finish(NrcState &N, cudaStream_t st, float *loss);
 // Gradient of the mean relative-L2 loss (times the loss scale) into N.g.
 kgk_status nrc_grad_dev(NrcState &N, const float *raw, int raw_stride, const float *tgt, int tgt_stride, int n,
                         const int *n_dev, cudaStream_t st);
-// Adam step from N.g (skipped when the gradient is not finite).
+// Adam step from N.g (skipped when the gradient is not finite or its kernels gave
+// up a wait).
 kgk_status nrc_step_dev(NrcState &N, cudaStream_t st);
 
 NrcState *nrc_state(kgk_scene *s);

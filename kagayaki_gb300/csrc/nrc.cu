@@ -524,9 +524,9 @@ __global__ void __launch_bounds__(tc::Ti<W>::kTileThreads * tc::Ti<W>::kGroups, 
 // reads, by the threads); the rows of the last tile past the sample count
 // are written too, with dY = 0.  Every mbarrier wait is bounded; a
 // timeout sets *err and ends the CTA after a last bounded wait for its MMAs,
-// freeing its tensor memory.
+// freeing its tensor memory.  kGiveUp: as k_infer_tc's.
 // ---------------------------------------------------------------------------
-template <int W>
+template <int W, bool kGiveUp>
 __global__ void __launch_bounds__(tc::Ti<W>::kTileThreads * tc::Tc<W>::kGroups) k_train_fb_tc(
     const unsigned short *__restrict__ img, const float *__restrict__ raw, int raw_stride,
     const float *__restrict__ target, int tgt_stride, int n, const int *n_dev, const float *scale_p,
@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(tc::Ti<W>::kTileThreads * tc::Tc<W>::kGroups) 
                 bulk_commit();
             }
         }
-        const bool ok = bar_wait(bar, phase);
+        const bool ok = !kGiveUp && bar_wait(bar, phase);
         phase ^= 1u;
         if (first && map) bulk_wait_read();  // the tile may be overwritten after the barrier below
         if (tile_sync_or<kTile>(wgbar, !ok)) return false;
@@ -830,7 +830,7 @@ __device__ __forceinline__ void tma_load3(uint32_t dst, const CUtensorMap *map, 
 }
 }  // namespace dwt
 
-template <int W>
+template <int W, bool kGiveUp>
 __global__ void __launch_bounds__(128) k_train_dw_tc(const __grid_constant__ CUtensorMap tmH,
                                                      const __grid_constant__ CUtensorMap tmD, int n,
                                                      const int *n_dev, int chunk, float *dW_glob, int *err) {
@@ -875,7 +875,7 @@ __global__ void __launch_bounds__(128) k_train_dw_tc(const __grid_constant__ CUt
         int issued = 0;
         for (int i = 0; i < nst; ++i) {
             const int s = i % S;
-            if (i >= S && !bar_wait(emptyb + 8u * s, (uint32_t)((i / S) - 1) & 1u)) {
+            if (i >= S && (kGiveUp || !bar_wait(emptyb + 8u * s, (uint32_t)((i / S) - 1) & 1u))) {
                 atomicExch(&failed_sh, 1);
                 break;
             }
@@ -896,7 +896,7 @@ __global__ void __launch_bounds__(128) k_train_dw_tc(const __grid_constant__ CUt
         const uint32_t lboA = ma == 2 ? dwt::kBox : 0u, lboB = nb == 2 ? dwt::kBox : 0u;
         for (int i = 0; i < nst; ++i) {
             const int s = i % S;
-            if (!bar_wait(fullb + 8u * s, (uint32_t)(i / S) & 1u)) {
+            if (kGiveUp || !bar_wait(fullb + 8u * s, (uint32_t)(i / S) & 1u)) {
                 atomicExch(&failed_sh, 1);
                 break;
             }
@@ -962,11 +962,14 @@ __global__ void k_make_image(const float *w, unsigned short *img) {
 // that all gradients are finite (n <= 74,112 floats, read from L2), block 0
 // records the verdict for k_scale_update, and if it is clean each updated
 // master weight is written to the image too (the image's padding never
-// changes).
+// changes).  No step, and no change of scale, on a gradient whose kernels gave up
+// a wait (*err): parts of it are missing.
 template <int W>
 __global__ void k_adam_image(float *w, float *m, float *v, const float *g, const float *scale_p, float lr, float b1,
-                             float b2, float eps, float bc1, float bc2, unsigned short *img, int *bad_out) {
+                             float b2, float eps, float bc1, float bc2, unsigned short *img, int *bad_out,
+                             const int *err) {
     constexpr int n = Net<W>::kParams, P = Net<W>::kPitch;
+    if (*err) return;
     int local = 0;
     for (int i = threadIdx.x; i < n; i += blockDim.x)
         if (!isfinite(g[i])) local = 1;
@@ -1003,7 +1006,8 @@ __global__ void k_adam_image(float *w, float *m, float *v, const float *g, const
 
 // Dynamic loss scaling: halve on a non-finite gradient, double after
 // kScaleGrowth clean steps.
-__global__ void k_scale_update(float *scale, int *good, const int *bad) {
+__global__ void k_scale_update(float *scale, int *good, const int *bad, const int *err) {
+    if (*err) return;
     if (*bad) {
         *scale = fmaxf(*scale * 0.5f, 1.0f);
         *good = 0;
@@ -1038,6 +1042,16 @@ void launch_infer(NrcState &N, const float *raw, int stride, int n, const int *n
     using I = tc::Ti<W>;
     auto *k = N.cfg.give_up_waits ? k_infer_tc<W, true> : k_infer_tc<W, false>;
     k<<<N.sms, I::kTileThreads * I::kGroups, I::kSmemBytes, st>>>(N.img, raw, stride, n, n_dev, out, rad, N.ints + 2);
+}
+
+// Shared memory beyond 48 KB for the kernels of a width.
+template <int W, bool kGiveUp>
+kgk_status set_smem() {
+    constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    KGK_CUDA(cudaFuncSetAttribute(k_train_dw_tc<W, kGiveUp>, kAttr, (int)dwt::Cfg<W>::kSmem));
+    KGK_CUDA(cudaFuncSetAttribute(k_train_fb_tc<W, kGiveUp>, kAttr, (int)tc::Tc<W>::kSmemBytes));
+    KGK_CUDA(cudaFuncSetAttribute(k_infer_tc<W, kGiveUp>, kAttr, (int)tc::Ti<W>::kSmemBytes));
+    return KGK_OK;
 }
 
 // cuTensorMapEncodeTiled, through the runtime's driver entry point.
@@ -1081,14 +1095,16 @@ kgk_status launch_grad(NrcState &N, const float *raw, int raw_stride, const floa
     KGK_TRY(scratch_map(&md, N.trD, W, N.tr_cap));
     // as many CTAs as the batch's 128-row tiles need (one per warpgroup), at most the resident count
     const int fb_ctas = std::max(1, std::min(N.sms * T::kCtasPerSm, ((n + 127) / 128 + T::kGroups - 1) / T::kGroups));
-    k_train_fb_tc<W><<<fb_ctas, tc::Ti<W>::kTileThreads * T::kGroups, T::kSmemBytes, st>>>(
+    auto *fb = N.cfg.give_up_waits ? k_train_fb_tc<W, true> : k_train_fb_tc<W, false>;
+    fb<<<fb_ctas, tc::Ti<W>::kTileThreads * T::kGroups, T::kSmemBytes, st>>>(
         N.img, raw, raw_stride, tgt, tgt_stride, n, n_dev, N.scal, N.trD, ls, mh, md, N.scal + 1, N.ints + 2);
     // split K: chunks of whole 64-row boxes, about two CTAs per SM over the six layers
     const int want = std::max(1, 2 * N.sms / (kLayers + 1));
     int chunk = std::max(1024, (rows + want - 1) / want);
     chunk = (chunk + 63) & ~63;
     const dim3 gdw((unsigned)((rows + chunk - 1) / chunk), kLayers + 1);
-    k_train_dw_tc<W><<<gdw, 128, dwt::Cfg<W>::kSmem, st>>>(mh, md, n, n_dev, chunk, N.g, N.ints + 2);
+    auto *dw = N.cfg.give_up_waits ? k_train_dw_tc<W, true> : k_train_dw_tc<W, false>;
+    dw<<<gdw, 128, dwt::Cfg<W>::kSmem, st>>>(mh, md, n, n_dev, chunk, N.g, N.ints + 2);
     return KGK_OK;
 }
 }  // namespace
@@ -1112,8 +1128,8 @@ kgk_status nrc_init(NrcState &N, const kgk_nrc_config *cfg, int device) {
     KGK_TRY(dalloc(&N.v, (size_t)N.params, "cache Adam state"));
     KGK_TRY(dalloc(&N.g, (size_t)N.params, "cache gradient"));
     KGK_TRY(dalloc(&N.img, (size_t)img_elems_of(W), "cache BF16 weights"));
-    KGK_TRY(dalloc(&N.scal, 4, "cache scalars"));
-    KGK_TRY(dalloc(&N.ints, 4, "cache scalars"));
+    KGK_TRY(dalloc(&N.scal, 8, "cache scalars"));
+    N.ints = reinterpret_cast<int *>(N.scal + 4);
     // He-uniform initialisation (bound sqrt(6 / inputs of the layer)) from a
     // seeded stream
     std::vector<float> h(N.params);
@@ -1135,23 +1151,12 @@ kgk_status nrc_init(NrcState &N, const kgk_nrc_config *cfg, int device) {
     make_image(N, 0);
     KGK_CUDA(cudaGetLastError());
     KGK_CUDA(cudaDeviceSynchronize());
-    KGK_CUDA(cudaFuncSetAttribute(k_train_dw_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)dwt::Cfg<64>::kSmem));
-    KGK_CUDA(cudaFuncSetAttribute(k_train_dw_tc<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)dwt::Cfg<128>::kSmem));
-    KGK_CUDA(cudaFuncSetAttribute(k_train_fb_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)tc::Tc<64>::kSmemBytes));
-    KGK_CUDA(cudaFuncSetAttribute(k_train_fb_tc<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)tc::Tc<128>::kSmemBytes));
-    KGK_CUDA(cudaFuncSetAttribute(k_infer_tc<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)tc::Ti<64>::kSmemBytes));
-    KGK_CUDA(cudaFuncSetAttribute(k_infer_tc<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)tc::Ti<128>::kSmemBytes));
     if (N.cfg.give_up_waits) {
-        KGK_CUDA(cudaFuncSetAttribute(k_infer_tc<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)tc::Ti<64>::kSmemBytes));
-        KGK_CUDA(cudaFuncSetAttribute(k_infer_tc<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)tc::Ti<128>::kSmemBytes));
+        if (W == 128) KGK_TRY((set_smem<128, true>()));
+        else KGK_TRY((set_smem<64, true>()));
+    } else {
+        if (W == 128) KGK_TRY((set_smem<128, false>()));
+        else KGK_TRY((set_smem<64, false>()));
     }
     cudaDeviceProp p;
     KGK_CUDA(cudaGetDeviceProperties(&p, device));
@@ -1162,7 +1167,7 @@ kgk_status nrc_init(NrcState &N, const kgk_nrc_config *cfg, int device) {
 }
 
 void nrc_free(NrcState &N) {
-    void *ptrs[] = {N.w, N.m, N.v, N.g, N.img, N.scal, N.ints, N.trH, N.trD};
+    void *ptrs[] = {N.w, N.m, N.v, N.g, N.img, N.scal, N.trH, N.trD};
     for (void *p : ptrs) dfree(p);
     N.w = N.m = N.v = N.g = N.scal = nullptr;
     N.img = N.trH = N.trD = nullptr;
@@ -1171,13 +1176,19 @@ void nrc_free(NrcState &N) {
     N.ready = false;
 }
 
-kgk_status nrc_check_error(NrcState &N) {
-    int e = 0;
-    KGK_CUDA(cudaMemcpy(&e, N.ints + 2, sizeof(int), cudaMemcpyDeviceToHost));
-    if (e) {
-        KGK_CUDA(cudaMemset(N.ints + 2, 0, sizeof(int)));
-        return fail(KGK_ERR_DEVICE_CHECK, "radiance cache: a tensor-core wait timed out (inference abandoned)");
+kgk_status nrc_finish(NrcState &N, cudaStream_t st, float *loss) {
+    struct {
+        float scal[4];
+        int ints[4];
+    } h;
+    KGK_CUDA(cudaMemcpyAsync(&h, N.scal, sizeof h, cudaMemcpyDeviceToHost, st));
+    KGK_CUDA(cudaStreamSynchronize(st));
+    if (h.ints[2]) {
+        // on the kernels' own stream: a late clear could wipe what the next call raises
+        KGK_CUDA(cudaMemsetAsync(N.ints + 2, 0, sizeof(int), st));
+        return fail(KGK_ERR_DEVICE_CHECK, "radiance cache: a tensor-core wait timed out (the call's results are void)");
     }
+    if (loss) *loss = h.scal[1];
     return KGK_OK;
 }
 
@@ -1225,11 +1236,11 @@ kgk_status nrc_step_dev(NrcState &N, cudaStream_t st) {
     // then the loss scale from block 0's verdict in N.ints[0]
     if (N.cfg.width == 128)
         k_adam_image<128><<<64, 256, 0, st>>>(N.w, N.m, N.v, N.g, N.scal, N.cfg.learning_rate, b1, b2, 1e-10f, bc1,
-                                              bc2, N.img, N.ints);
+                                              bc2, N.img, N.ints, N.ints + 2);
     else
         k_adam_image<64><<<64, 256, 0, st>>>(N.w, N.m, N.v, N.g, N.scal, N.cfg.learning_rate, b1, b2, 1e-10f, bc1,
-                                             bc2, N.img, N.ints);
-    k_scale_update<<<1, 1, 0, st>>>(N.scal, N.ints + 1, N.ints);
+                                             bc2, N.img, N.ints, N.ints + 2);
+    k_scale_update<<<1, 1, 0, st>>>(N.scal, N.ints + 1, N.ints, N.ints + 2);
     KGK_CUDA(cudaGetLastError());
     return KGK_OK;
 }
@@ -1324,8 +1335,7 @@ kgk_status kgk_nrc_infer(kgk_scene *s, const float *raw, size_t n, float *out) {
     }
     KGK_TRY(nrc_infer_dev(*s->nrc, (const float *)draw, kRaw, (int)n, nullptr, (float *)dout, nullptr, s->stream));
     if (!od) KGK_CUDA(cudaMemcpyAsync(out, dout, n * 3 * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
-    KGK_CUDA(cudaStreamSynchronize(s->stream));
-    return nrc_check_error(*s->nrc);
+    return nrc_finish(*s->nrc, s->stream, nullptr);
 }
 
 kgk_status kgk_nrc_gradients(kgk_scene *s, const float *raw, const float *target, size_t n, float *grad, float *loss) {
@@ -1346,11 +1356,7 @@ kgk_status kgk_nrc_gradients(kgk_scene *s, const float *raw, const float *target
     k_unscale<<<64, 256, 0, s->stream>>>(N.g, N.params, N.scal, (float *)dg);
     KGK_CUDA(cudaGetLastError());
     KGK_CUDA(cudaMemcpyAsync(grad, dg, N.params * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
-    float hl = 0.0f;
-    KGK_CUDA(cudaMemcpyAsync(&hl, N.scal + 1, sizeof(float), cudaMemcpyDeviceToHost, s->stream));
-    KGK_CUDA(cudaStreamSynchronize(s->stream));
-    if (loss) *loss = hl;
-    return KGK_OK;
+    return nrc_finish(N, s->stream, loss);
 }
 
 kgk_status kgk_nrc_train(kgk_scene *s, const float *raw, const float *target, size_t n, int32_t steps, float *loss) {
@@ -1367,11 +1373,7 @@ kgk_status kgk_nrc_train(kgk_scene *s, const float *raw, const float *target, si
         KGK_TRY(nrc_grad_dev(N, (const float *)draw, kRaw, (const float *)dt, 3, (int)n, nullptr, s->stream));
         KGK_TRY(nrc_step_dev(N, s->stream));
     }
-    float hl = 0.0f;
-    KGK_CUDA(cudaMemcpyAsync(&hl, N.scal + 1, sizeof(float), cudaMemcpyDeviceToHost, s->stream));
-    KGK_CUDA(cudaStreamSynchronize(s->stream));
-    if (loss) *loss = hl;
-    return KGK_OK;
+    return nrc_finish(N, s->stream, loss);
 }
 
 kgk_status kgk_nrc_loss_scale(kgk_scene *s, float *scale) {

@@ -2115,7 +2115,7 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
         stats->rays_tail = hs[kRaysT];
     }
     for (cudaEvent_t e : ev) cudaEventDestroy(e);
-    if (cfg->use_cache) KGK_TRY(nrc_check_error(*s->nrc));
+    if (cfg->use_cache) KGK_TRY(nrc_finish(*s->nrc, st, nullptr));
     if (hs[kOverflow])
         return fail(KGK_ERR_DEVICE_CHECK, "kgk_render: " + std::to_string(hs[kOverflow]) +
                                               " traversals overflowed their stack");
