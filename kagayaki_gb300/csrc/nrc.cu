@@ -1303,7 +1303,10 @@ kgk_status kgk_nrc_set_weights(kgk_scene *s, const float *w, size_t n) {
     NrcState &N = *s->nrc;
     if (!w || n != (size_t)N.params)
         return fail(KGK_ERR_INVALID_ARGUMENT, "kgk_nrc_set_weights: expected " + std::to_string(N.params) + " floats");
+    // On the legacy stream, after what made the weights there; the host may be back
+    // before the copy is done, and the scene's stream does not wait for that one.
     KGK_CUDA(cudaMemcpy(N.w, w, n * sizeof(float), is_device_ptr(w) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
+    KGK_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     make_image(N, s->stream);
     KGK_CUDA(cudaGetLastError());
     KGK_CUDA(cudaStreamSynchronize(s->stream));
@@ -1317,6 +1320,7 @@ kgk_status kgk_nrc_get_weights(kgk_scene *s, float *w, size_t n) {
                     "kgk_nrc_get_weights: expected " + std::to_string(s->nrc->params) + " floats");
     KGK_CUDA(cudaStreamSynchronize(s->stream));
     KGK_CUDA(cudaMemcpy(w, s->nrc->w, n * sizeof(float), is_device_ptr(w) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost));
+    KGK_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // before a later step changes them
     return KGK_OK;
 }
 
