@@ -255,6 +255,9 @@ kgk_status scene_upload(DevScene &s, const kgk_triangle *tris_in, size_t n, cons
             KGK_CUDA(cudaMemcpy(s.tex_pixels + desc[i].offset, th[i].pixels, cnt * sizeof(float),
                                 is_device_ptr(th[i].pixels) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
         }
+        // the host may be back before the copies are done, and `st` does not wait
+        // for the legacy stream, on which they are (after what made the texels)
+        KGK_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
         KGK_TRY(upload(&s.tex, desc.data(), ntex, "texture table", st));
         s.n_tex = (int32_t)ntex;
     }
@@ -358,6 +361,7 @@ kgk_status scene_set_textures_rgba8(DevScene &s, const kgk_texture_rgba8 *tex, s
         KGK_CUDA(cudaMemcpy(s.tex_rgba8 + desc[i].offset, tex[i].pixels, cnt * 4,
                             is_device_ptr(tex[i].pixels) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
     }
+    KGK_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // as in the scene's creation
     if (!s.tex_lut) {
         float lut[256];
         for (int v = 0; v < 256; ++v) lut[v] = (float)((double)powf(v / 255.0f, 2.2f) + 1e-4);

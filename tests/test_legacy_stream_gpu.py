@@ -50,3 +50,54 @@ def test_cache_weights(width):
         check(lib().kgk_nrc_get_weights(s._h, _p(back), n))
         check(lib().kgk_nrc_train(s._h, _p(raw), _p(tgt), 1000, 1, None))
         assert np.array_equal(back.cpu().numpy(), w)
+
+
+@pytest.mark.parametrize("rgba8", [False, True])
+def test_textures(rgba8):
+    import test_texture_gpu as T
+    from kagayaki_gb300 import ESTIMATOR_UNBIASED, camera_setup
+    from kagayaki_gb300.structs import KgkTexture, KgkTextureRGBA8
+    rng = np.random.default_rng(5)
+    if rgba8:
+        tex = rng.integers(0, 256, (256, 256, 4), np.uint8)
+        make, args = KgkTextureRGBA8, (256, 256)
+    else:
+        tex = rng.random((256, 256, 3), dtype=np.float32)
+        make, args = KgkTexture, (256, 256, 3)
+    tris, mats = T.quad_scene()
+    env = np.ones((16, 32, 3), np.float32)
+    cam = camera_setup((0.0, 0.0, 3.0), 28.0, (0.0, 0.0, 0.0), 64)
+
+    def frame(s):
+        s.build_bvh()
+        return s.render(cam, 64, 64, spp=4, estimator=ESTIMATOR_UNBIASED, seed=5, max_depth=3)[0].copy()
+
+    placeholder = [np.zeros((1, 1, 3), np.float32)]
+    with Scene(tris, mats, textures=placeholder if rgba8 else [tex], env=env) as s:
+        if rgba8:
+            s.set_textures_rgba8([tex])
+        want = frame(s)
+    host = torch.from_numpy(tex).pin_memory()
+    dev = torch.zeros_like(host, device="cuda")
+    torch.cuda.synchronize()
+    t = make()
+    t.pixels = ctypes.cast(dev.data_ptr(), type(t.pixels)) if not rgba8 else dev.data_ptr()
+    t.width, t.height = args[:2]
+    if rgba8:
+        with Scene(tris, mats, textures=placeholder, env=env) as s:
+            keep_busy()
+            dev.copy_(host, non_blocking=True)
+            check(lib().kgk_scene_set_textures_rgba8(s._h, ctypes.byref(t), 1))
+            got = frame(s)
+    else:
+        t.bpp = 3
+        hdr = KgkTexture(env.ctypes.data_as(ctypes.POINTER(ctypes.c_float)), 32, 16, 3)
+        s = Scene.__new__(Scene)
+        s._h, s.bvh = ctypes.c_void_p(), None
+        keep_busy()
+        dev.copy_(host, non_blocking=True)
+        check(lib().kgk_scene_create(_p(tris), len(tris), _p(mats), len(mats), ctypes.byref(t), 1, ctypes.byref(hdr),
+                                     ctypes.byref(s._h)))
+        got = frame(s)
+        s.close()
+    assert np.array_equal(got, want)
