@@ -145,7 +145,8 @@ typedef struct kgk_stats {
     uint64_t rays_shadow;         /* shadow / occlusion rays                     */
     uint64_t traversal_overflows; /* rays whose traversal stack overflowed      */
     uint64_t nodes_visited;       /* wide nodes intersected by the wavefront's closest-hit
-                                     rays (count_work only; not the tail kernel's) */
+                                     rays (count_work only; not the tail kernel's, so 0 for
+                                     waves of at most 131,072 paths) */
     uint64_t tris_tested;         /* triangles tested, likewise                 */
     uint64_t paths;               /* camera paths traced                         */
     double ms_device;             /* device time of the call (CUDA events)       */
@@ -154,8 +155,10 @@ typedef struct kgk_stats {
     double ms_shade;              /* shading stage device time (profile_stages)  */
     double ms_shadow;             /* shadow-ray stage device time (profile_stages) */
     uint64_t extend_launches;     /* closest-hit (extend) kernel launches        */
-    double ms_tail;               /* tail-kernel device time (profile_stages)    */
-    uint64_t rays_tail;           /* closest-hit rays traced by the tail kernel (part of rays_closest) */
+    double ms_tail;               /* device time of the kernels that take paths from start to
+                                     end (profile_stages): the tail kernel, and the one that
+                                     renders small compat scenes and images a pixel per thread */
+    uint64_t rays_tail;           /* closest-hit rays traced by those kernels (part of rays_closest) */
 } kgk_stats;
 
 typedef struct kgk_bvh_info {

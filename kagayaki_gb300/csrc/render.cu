@@ -1875,8 +1875,10 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
     // at 36 triangles (0.80 : 1.77 with Disney boxes), 1.05 : 0.98 at 2,562,
     // 1.25 : 1.16 at 5,122, 2.8 : 2.0 at 1.3M.  Two rounds of one block per SM
     // at most: 400 x 400 1.14 : 1.43 ms, 640 x 480 1.98 : 1.71.
+    // Not where the caller wants nodes and triangles counted and a wave would do
+    // it (one that does not start in the tail kernel).
     const bool by_pixel = cfg->estimator == KGK_ESTIMATOR_COMPAT && s->dev.n_tris <= kCompatTris &&
-                          npx <= 2 * kCompatThreads * R.sms;
+                          npx <= 2 * kCompatThreads * R.sms && !(cfg->count_work && npx > kTailPaths);
     if (by_pixel) {
         P.spp_wave = 1;
         // one block per SM, whose warps are then all in step

@@ -1,0 +1,37 @@
+"""The reference's estimator on small scenes, where it changes between a pixel
+per thread and waves: what a call reports and renders does not depend on the way
+it takes."""
+import numpy as np
+import pytest
+
+from kagayaki_gb300 import ESTIMATOR_COMPAT, Scene, camera_setup, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def rendered(n_far, W, H, spp, **kw):
+    from test_compat_routes_gpu import far_away
+    tris, mats, c, tex, env = scenes.parity_scene("cornell")
+    with Scene(far_away(tris, n_far), mats, textures=tex, env=env) as s:
+        s.build_bvh()
+        s.accum_reset(W, H)
+        cam = camera_setup(c["origin"], c["dist"], c["rot"], H)
+        img, st = s.render(cam, W, H, spp=spp, estimator=ESTIMATOR_COMPAT, accumulate=True, **kw)
+        return img.copy(), st, s.accum_read(W, H)
+
+
+def same(a, b):
+    assert np.array_equal(a[0], b[0], equal_nan=True)
+    assert all(np.array_equal(x, y, equal_nan=True) for x, y in zip(a[2], b[2]))
+    assert [a[1][k] for k in ("rays_closest", "rays_shadow", "paths")] == \
+           [b[1][k] for k in ("rays_closest", "rays_shadow", "paths")]
+
+
+@pytest.mark.parametrize("W,H", [(363, 362), (400, 380), (450, 450)])
+def test_work_is_counted_above_the_tail_kernels_waves(W, H):
+    plain, counted = rendered(0, W, H, 2), rendered(0, W, H, 2, count_work=True)
+    same(plain, counted)
+    st = counted[1]
+    assert st["extend_launches"] >= 2
+    assert st["nodes_visited"] >= st["rays_closest"] - st["rays_tail"] > 0
+    assert st["tris_tested"] > 0
