@@ -118,8 +118,10 @@ enum Stat { kRaysC = 0, kRaysS = 1, kOverflow = 2, kNodes = 3, kTris = 4, kRaysT
 constexpr int kTailPaths = 1 << 17;
 // Idle lanes of a tail warp that take new paths together.
 constexpr int kTailRefill = 8;
-// k_compat: the largest scene it renders and its threads per block.
-constexpr int kCompatTris = 1024, kCompatThreads = 512;
+// k_compat: the largest scene it renders, its threads per block, and the samples
+// of a launch, so that a call of many leaves the GPU to others in between (64
+// take 8 to 20 ms; a wave per sample did after each).
+constexpr int kCompatTris = 1024, kCompatThreads = 512, kCompatSamples = 64;
 // The largest scene whose waves trace by k_extend_loop and k_shadow_loop.
 constexpr int kLoopTris = 1024;
 // Deferred shadow rays of the tail (unbiased estimator without the cache):
@@ -1316,20 +1318,21 @@ __device__ __forceinline__ void compat_flush(const Params &P, const CompatCount 
 }
 
 // A pixel per thread (slots in 8 x 4 tiles), the block going through the
-// call's samples one after another.  The seed chain orders a pixel's own
+// launch's samples one after another; `first`: of the call, else the frame's sums
+// go on.  The seed chain orders a pixel's own
 // samples only (render.cuh:19,29,42), so no block waits for another's longest
 // path and a sample needs no launches.  Cornell box, 256 x 256, 16 samples:
 // 3.36 -> 2.44 ms (a wave of three launches per sample before; the same with
 // a barrier per phase 2.81; a warp going through its 32 pixels' samples alone
 // 3.30).
 __global__ void __launch_bounds__(kCompatThreads) k_compat(Params P, int spp, int bounces, float4 *frame, double *acc_sum,
-                                                double *acc_sq, int accumulate) {
+                                                double *acc_sq, int accumulate, int first) {
     CompatCount c;
     for (int base = blockIdx.x * blockDim.x; base < P.npx; base += gridDim.x * blockDim.x) {
         const int slot = base + threadIdx.x;
         const bool mine = slot < P.npx;
         const int px = mine ? tiled_path(P, slot) : 0;
-        float3 f = f3(0.0f, 0.0f, 0.0f);
+        float3 f = mine && !first ? f3(frame[px]) : f3(0.0f, 0.0f, 0.0f);
 #pragma unroll 1
         for (int smp = 0; smp < spp; ++smp) {
             PathState ps;
@@ -1869,7 +1872,7 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
         return KGK_OK;
     };
     // The reference's estimator on a small scene and image: a pixel per thread,
-    // all samples in one launch (k_compat).  The block goes at the pace of its
+    // up to kCompatSamples samples in a launch (k_compat).  The block goes at the pace of its
     // longest traversal, so only while the tree is a few nodes: measured
     // against the wave per sample, 256 x 256 pixels, 4 samples, 0.60 : 0.82 ms
     // at 36 triangles (0.80 : 1.77 with Disney boxes), 1.05 : 0.98 at 2,562,
@@ -1883,12 +1886,14 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
         P.spp_wave = 1;
         // one block per SM, whose warps are then all in step
         const int per = std::min(kCompatThreads, std::max(32, ((npx + R.sms - 1) / R.sms + 31) & ~31));
-        KGK_TRY(stage_begin(3));
-        k_compat<<<(npx + per - 1) / per, per, 0, st>>>(P, cfg->spp, max_bounces, R.frame, R.acc_sum, R.acc_sq,
-                                                        cfg->accumulate);
-        KGK_TRY(stage_end());
-        KGK_CUDA(cudaGetLastError());
-        ++launches;
+        for (int done = 0; done < cfg->spp; done += kCompatSamples) {
+            KGK_TRY(stage_begin(3));
+            k_compat<<<(npx + per - 1) / per, per, 0, st>>>(P, std::min(kCompatSamples, cfg->spp - done), max_bounces,
+                                                            R.frame, R.acc_sum, R.acc_sq, cfg->accumulate, done == 0);
+            KGK_TRY(stage_end());
+            KGK_CUDA(cudaGetLastError());
+            ++launches;
+        }
     }
     // trees of a few nodes: rays by the one-ray loops.  Loops : pairs, the
     // reference's estimator at 640 x 480 x 4 / the unbiased at 1080p x 8, ms:

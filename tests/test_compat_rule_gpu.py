@@ -35,3 +35,14 @@ def test_work_is_counted_above_the_tail_kernels_waves(W, H):
     assert st["extend_launches"] >= 2
     assert st["nodes_visited"] >= st["rays_closest"] - st["rays_tail"] > 0
     assert st["tris_tested"] > 0
+
+
+def test_samples_of_a_launch():
+    """64 samples a launch: the same sums as a wave per sample, and no launch holds
+    the GPU for a whole call of many."""
+    launches = []
+    for spp in (64, 65, 130):
+        got = rendered(0, 33, 31, spp)
+        same(got, rendered(2000, 33, 31, spp))
+        launches.append(got[1]["kernel_launches"])
+    assert [n - launches[0] for n in launches] == [0, 1, 2]
