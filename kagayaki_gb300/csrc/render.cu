@@ -122,6 +122,8 @@ constexpr int kTailRefill = 8;
 // of a launch, so that a call of many leaves the GPU to others in between (64
 // take 8 to 20 ms; a wave per sample did after each).
 constexpr int kCompatTris = 1024, kCompatThreads = 512, kCompatSamples = 64;
+// ... and the largest scene of which it renders one or two samples of a small image.
+constexpr int kCompatFewTris = 128;
 // The largest scene whose waves trace by k_extend_loop and k_shadow_loop.
 constexpr int kLoopTris = 1024;
 // Deferred shadow rays of the tail (unbiased estimator without the cache):
@@ -413,9 +415,9 @@ __global__ void __launch_bounds__(128, 8) k_extend(Params P, int cnt_idx, int de
 // through the one-ray loops: with up to 24 triangles in a node and nodes that
 // nearly every ray enters, the lanes' own lists are alike, and an occluded ray
 // leaves its list at once.  Instruction issue bounds them.  640 x 480, the
-// reference's estimator, 4 samples: 1.74 -> 1.57 ms on the 36-triangle box, 2.07
+// reference's estimator, 4 samples: 1.73 -> 1.54 ms on the 36-triangle box, 2.08
 // -> 1.89 with Disney boxes; 82 triangles, 1080p, 8 samples of the unbiased one:
-// 3.72 -> 3.31 ms.
+// 3.71 -> 3.28 ms.
 template <bool kCount>
 __global__ void __launch_bounds__(128, 8) k_extend_loop(Params P, int cnt_idx, int dense_n, int *mq, int *lq, int *dq) {
     const int n = cnt_idx >= 0 ? P.cnt[cnt_idx] : dense_n;
@@ -1872,16 +1874,28 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
         return KGK_OK;
     };
     // The reference's estimator on a small scene and image: a pixel per thread,
-    // up to kCompatSamples samples in a launch (k_compat).  The block goes at the pace of its
-    // longest traversal, so only while the tree is a few nodes: measured
-    // against the wave per sample, 256 x 256 pixels, 4 samples, 0.60 : 0.82 ms
-    // at 36 triangles (0.80 : 1.77 with Disney boxes), 1.05 : 0.98 at 2,562,
-    // 1.25 : 1.16 at 5,122, 2.8 : 2.0 at 1.3M.  Two rounds of one block per SM
-    // at most: 400 x 400 1.14 : 1.43 ms, 640 x 480 1.98 : 1.71.
+    // up to kCompatSamples samples in a launch (k_compat).  The block goes at the
+    // pace of its longest traversal, so only while the tree is a few nodes.
+    // Measured against a wave per sample as below, ms, of the scenes named by their
+    // triangles (36: the box, 36d: with Disney boxes):
+    //   256 x 256 x 4    36 0.60 : 0.77, 36d 0.79 : 1.25, 82 0.61 : 0.65, 642 0.80 : 0.82,
+    //                    962 0.81 : 0.81, 1,282 0.83 : 0.86, 2,562 1.05 : 0.92 to 1.17 : 1.02
+    //   316 x 316 x 4    36 1.07 : 1.09, 36d 1.37 : 1.76, 642 0.70 : 0.78, 2,562 1.08 : 1.13
+    //   400 x 400 x 4    36 1.14 : 1.32, 36d 1.46 : 1.71, 642 0.88 : 1.20
+    // One and two samples do not pay for the barriers on more than a few nodes as
+    // long as a wave is the tail kernel's: 256 x 256, 1 and 2 samples, 82 0.155 : 0.162
+    // and 0.305 : 0.324, 162 0.162 : 0.157 and 0.315 : 0.316, 322 0.209 : 0.195 and
+    // 0.384 : 0.380, 642 0.205 : 0.187 and 0.437 : 0.412; larger waves are behind again
+    // (400 x 400, 642: 0.244 : 0.302 and 0.432 : 0.593).
+    // Blocks go round the SMs; a third round that is not nearly empty costs more
+    // than it gives on the box: 169,744 pixels 0.308 : 0.341 (36) and 0.386 : 0.436
+    // (36d), 174,724 0.398 : 0.347 and 0.501 : 0.447.
     // Not where the caller wants nodes and triangles counted and a wave would do
     // it (one that does not start in the tail kernel).
     const bool by_pixel = cfg->estimator == KGK_ESTIMATOR_COMPAT && s->dev.n_tris <= kCompatTris &&
-                          npx <= 2 * kCompatThreads * R.sms && !(cfg->count_work && npx > kTailPaths);
+                          npx <= kCompatThreads * (2 * R.sms + R.sms / 6) &&
+                          (cfg->spp > 2 || s->dev.n_tris <= kCompatFewTris || npx > kTailPaths) &&
+                          !(cfg->count_work && npx > kTailPaths);
     if (by_pixel) {
         P.spp_wave = 1;
         // one block per SM, whose warps are then all in step
@@ -1895,14 +1909,25 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
             ++launches;
         }
     }
-    // trees of a few nodes: rays by the one-ray loops.  Loops : pairs, the
-    // reference's estimator at 640 x 480 x 4 / the unbiased at 1080p x 8, ms:
-    // 642 triangles 1.38 : 1.38 / 3.6 : 3.85, 1,282 1.41 : 1.42 / 3.98 : 4.14,
-    // 2,562 1.59 : 1.54 / 3.68 : 3.85 and 1.44 : 1.42 / 5.1 : 5.0.
+    // Trees of a few nodes: rays by the one-ray loops.  Loops : pairs, ms, the
+    // reference's estimator at 640 x 480 x 4 / 1280 x 720 x 2, the unbiased one at
+    // 640 x 480 x 4 / 1080p x 8:
+    //   36     1.54 : 1.73, 1.33 : 1.44, 1.11 : 1.14, 7.77 : 7.96
+    //   82     1.06 : 1.10, 0.80 : 0.86, 0.59 : 0.63, 3.28 : 3.71
+    //   642    1.37 : 1.39, 0.95 : 0.98, 0.65 : 0.68, 3.51 : 3.87
+    //   962    1.35 : 1.35, 0.97 : 0.98, 0.75 : 0.75, 3.69 : 4.04
+    //   1,282  1.41 : 1.41, 0.99 : 1.00, 0.74 : 0.75, 3.84 : 4.13
+    //   2,562  1.44 : 1.39, 1.06 : 1.02, 0.80 : 0.76, 5.01 : 4.98 (spheres under a sky)
+    //          1.58 : 1.54, 1.08 : 1.05, 0.73 : 0.73, 3.60 : 3.95 (two spheres)
+    //          1.65 : 1.59, 1.15 : 1.12, 0.98 : 0.94, 4.66 : 4.69 (eight spheres)
+    // Even between 962 and 1,282 triangles, but for large unbiased waves.
     // Blocks of large waves finish at different times; three times what fits at
-    // once evens them out (1080p, reference's estimator, a sample a wave: 1.27 ->
-    // 1.245 ms on the box; unbiased, 8 samples: 8.03 -> 7.79 ms), but costs small
-    // waves (640 x 480: 1.56 -> 1.61 ms).
+    // once evens them out, but costs small ones.  Paths of a wave, one : three
+    // times, on the box: 0.31M 0.514 : 0.544 (unbiased), 1.54 : 1.59 (the
+    // reference's); 0.61M 0.720 : 0.717; 0.79M 1.43 : 1.44 (the reference's); 0.92M
+    // 0.793 : 0.790, 1.33 : 1.34; 1.23M 1.110 : 1.108; 1.31M 2.23 : 2.19 (the
+    // reference's); 1.84M 1.236 : 1.214; 2.07M 1.351 : 1.316, 2.52 : 2.48; 16.6M
+    // 8.01 : 7.77.
     const bool loops = s->dev.n_tris <= kLoopTris;
     const int loop_grid = (size_t)npx * std::min(spw, (int)cfg->spp) >= (1u << 20) ? 3 * grid : grid;
     auto shadow = [&](int q) {

@@ -46,3 +46,12 @@ def test_samples_of_a_launch():
         same(got, rendered(2000, 33, 31, spp))
         launches.append(got[1]["kernel_launches"])
     assert [n - launches[0] for n in launches] == [0, 1, 2]
+
+
+@pytest.mark.parametrize("n_tris,W,H,spp", [
+    (n, W, H, spp) for n, W, H in ((128, 97, 61), (129, 97, 61), (129, 363, 361), (129, 364, 361))
+    for spp in (1, 2, 3)] + [(36, 416, 404, 1), (36, 418, 403, 1)])
+def test_both_sides_of_the_lines(n_tris, W, H, spp):
+    """Triangles and samples, paths of a wave of the tail kernel (363 x 361 is the
+    last size), pixels: as with more triangles than the kernel takes."""
+    same(rendered(n_tris - 36, W, H, spp), rendered(2000, W, H, spp))
