@@ -8,7 +8,8 @@
 //   2. large tasks (> kSmall primitives): one level at a time, many blocks per
 //      task: 32-bin centroid binning per axis (shared-memory atomics merged
 //      into per-task global bins), one warp evaluates SAH over the 3 x 31
-//      planes, a chunked stable partition (block scans) reorders the refs;
+//      planes, a stable partition by chunks (warp ballots over the bin codes)
+//      reorders the refs;
 //   3. small tasks (<= kSmall): one block builds the whole subtree in shared
 //      memory, a warp per node, nodes of at most 32 primitives one primitive
 //      per lane; a split's place among the refs names its children's node

@@ -651,8 +651,8 @@ __global__ void __launch_bounds__(kRowT) k_c_atrous_rows(CompatArgs a, CompatIO 
     __syncthreads();
     const int x = blockIdx.x * T::T + threadIdx.x;
     if (x >= W) return;
-    constexpr int stage = kStep == 8 ? 3 : kStep == 16 ? 4 : kStep == 32 ? 5 : 6;
-    static_assert((1 << stage) == kStep, "row-tile steps are 8, 16, 32 and 64");
+    static_assert(kStep == 8 || kStep == 16, "the steps of stages 3 and 4");
+    constexpr int stage = kStep == 8 ? 3 : 4;
     const CompatRows<T::SX, kStep> S{s_nd, s_dm, s_mv, 2 * T::SX + (int)threadIdx.x + T::R};
     compat_atrous_px2(a, io, S, x, y, stage);
 }

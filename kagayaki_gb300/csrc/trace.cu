@@ -36,9 +36,10 @@ __device__ __forceinline__ void flush_counters(TraceCounters *ctr, unsigned node
 }
 
 // Lanes take new rays (one atomic per warp) whenever kRefill or more of them
-// are idle, so a warp does not wait for its longest ray; warp_step keeps the
-// same node and triangle order as trace_closest / trace_any, so the answers
-// are the same.
+// are idle, so a warp does not wait for its longest ray.  warp_step visits a
+// ray's nodes in trace_closest's / trace_any's order and tests the triangles of a
+// visit in the order of its pairs; the closest hit, ties by the smaller id, does not
+// depend on that, so the answers are the same.
 constexpr int kRefill = 8;
 
 template <bool kAny, bool kCount>
