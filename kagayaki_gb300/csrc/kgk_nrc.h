@@ -55,9 +55,15 @@ void nrc_free(NrcState &N);
 // floats 13..15 and the path id (int bits) at float 16 of each record.
 kgk_status nrc_infer_dev(NrcState &N, const float *raw, int stride, int n, const int *n_dev, float *out, float4 *rad,
                          cudaStream_t st);
-// Waits for the stream.  KGK_ERR_DEVICE_CHECK (and clears the flag) when a kernel
-// gave up a bounded wait; else *loss (may be null) is the last loss.
-kgk_status nrc_finish(NrcState &N, cudaStream_t st, float *loss);
+// The scalars as the stream's work leaves them: queue the copy with the call's
+// last work, and look at it after the wait for that.  nrc_status is
+// KGK_ERR_DEVICE_CHECK (and clears the flag) when a kernel gave up a bounded wait.
+struct NrcStatus {
+    float scal[4];
+    int ints[4];
+};
+kgk_status nrc_status_copy(NrcState &N, NrcStatus &h, cudaStream_t st);
+kgk_status nrc_status(NrcState &N, const NrcStatus &h, cudaStream_t st);
 // Gradient of the mean relative-L2 loss (times the loss scale) into N.g.
 kgk_status nrc_grad_dev(NrcState &N, const float *raw, int raw_stride, const float *tgt, int tgt_stride, int n,
                         const int *n_dev, cudaStream_t st);

@@ -969,13 +969,13 @@ __global__ void k_adam_image(float *w, float *m, float *v, const float *g, const
                              float b2, float eps, float bc1, float bc2, unsigned short *img, int *bad_out,
                              const int *err) {
     constexpr int n = Net<W>::kParams, P = Net<W>::kPitch;
-    if (*err) return;
+    const int gone = *err;  // looked at below, beside the gradients
     int local = 0;
     for (int i = threadIdx.x; i < n; i += blockDim.x)
         if (!isfinite(g[i])) local = 1;
     const int bad = __syncthreads_or(local);
     if (blockIdx.x == 0 && threadIdx.x == 0) *bad_out = bad;
-    if (bad) return;
+    if (bad || gone) return;
     const float inv_s = 1.0f / *scale_p;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float gi = g[i] * inv_s;
@@ -1007,8 +1007,9 @@ __global__ void k_adam_image(float *w, float *m, float *v, const float *g, const
 // Dynamic loss scaling: halve on a non-finite gradient, double after
 // kScaleGrowth clean steps.
 __global__ void k_scale_update(float *scale, int *good, const int *bad, const int *err) {
+    const int is_bad = *bad;
     if (*err) return;
-    if (*bad) {
+    if (is_bad) {
         *scale = fmaxf(*scale * 0.5f, 1.0f);
         *good = 0;
     } else if (++*good >= kScaleGrowth) {
@@ -1176,19 +1177,17 @@ void nrc_free(NrcState &N) {
     N.ready = false;
 }
 
-kgk_status nrc_finish(NrcState &N, cudaStream_t st, float *loss) {
-    struct {
-        float scal[4];
-        int ints[4];
-    } h;
+kgk_status nrc_status_copy(NrcState &N, NrcStatus &h, cudaStream_t st) {
     KGK_CUDA(cudaMemcpyAsync(&h, N.scal, sizeof h, cudaMemcpyDeviceToHost, st));
-    KGK_CUDA(cudaStreamSynchronize(st));
+    return KGK_OK;
+}
+
+kgk_status nrc_status(NrcState &N, const NrcStatus &h, cudaStream_t st) {
     if (h.ints[2]) {
         // on the kernels' own stream: a late clear could wipe what the next call raises
         KGK_CUDA(cudaMemsetAsync(N.ints + 2, 0, sizeof(int), st));
         return fail(KGK_ERR_DEVICE_CHECK, "radiance cache: a tensor-core wait timed out (the call's results are void)");
     }
-    if (loss) *loss = h.scal[1];
     return KGK_OK;
 }
 
@@ -1281,6 +1280,16 @@ struct Owned {
     }
 };
 
+// Waits for the call's work; *loss (may be null) is the last loss unless it failed.
+kgk_status finish(NrcState &N, cudaStream_t st, float *loss) {
+    NrcStatus h;
+    KGK_TRY(nrc_status_copy(N, h, st));
+    KGK_CUDA(cudaStreamSynchronize(st));
+    KGK_TRY(nrc_status(N, h, st));
+    if (loss) *loss = h.scal[1];
+    return KGK_OK;
+}
+
 kgk_status need(kgk_scene *s) {
     if (!s) return fail(KGK_ERR_INVALID_ARGUMENT, "radiance cache: scene == NULL");
     if (!s->nrc || !s->nrc->ready) return fail(KGK_ERR_INVALID_ARGUMENT, "radiance cache: call kgk_nrc_init first");
@@ -1339,7 +1348,7 @@ kgk_status kgk_nrc_infer(kgk_scene *s, const float *raw, size_t n, float *out) {
     }
     KGK_TRY(nrc_infer_dev(*s->nrc, (const float *)draw, kRaw, (int)n, nullptr, (float *)dout, nullptr, s->stream));
     if (!od) KGK_CUDA(cudaMemcpyAsync(out, dout, n * 3 * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
-    return nrc_finish(*s->nrc, s->stream, nullptr);
+    return finish(*s->nrc, s->stream, nullptr);
 }
 
 kgk_status kgk_nrc_gradients(kgk_scene *s, const float *raw, const float *target, size_t n, float *grad, float *loss) {
@@ -1360,7 +1369,7 @@ kgk_status kgk_nrc_gradients(kgk_scene *s, const float *raw, const float *target
     k_unscale<<<64, 256, 0, s->stream>>>(N.g, N.params, N.scal, (float *)dg);
     KGK_CUDA(cudaGetLastError());
     KGK_CUDA(cudaMemcpyAsync(grad, dg, N.params * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
-    return nrc_finish(N, s->stream, loss);
+    return finish(N, s->stream, loss);
 }
 
 kgk_status kgk_nrc_train(kgk_scene *s, const float *raw, const float *target, size_t n, int32_t steps, float *loss) {
@@ -1377,7 +1386,7 @@ kgk_status kgk_nrc_train(kgk_scene *s, const float *raw, const float *target, si
         KGK_TRY(nrc_grad_dev(N, (const float *)draw, kRaw, (const float *)dt, 3, (int)n, nullptr, s->stream));
         KGK_TRY(nrc_step_dev(N, s->stream));
     }
-    return nrc_finish(N, s->stream, loss);
+    return finish(N, s->stream, loss);
 }
 
 kgk_status kgk_nrc_loss_scale(kgk_scene *s, float *scale) {

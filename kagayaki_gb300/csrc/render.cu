@@ -2118,6 +2118,8 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
     if (!od) KGK_CUDA(cudaMemcpyAsync(out, dout, (size_t)npx * sizeof(float4), cudaMemcpyDeviceToHost, st));
     unsigned long long hs[kNStat];
     KGK_CUDA(cudaMemcpyAsync(hs, R.stats, sizeof hs, cudaMemcpyDeviceToHost, st));
+    NrcStatus cache_status;
+    if (cfg->use_cache) KGK_TRY(nrc_status_copy(*s->nrc, cache_status, st));
     KGK_CUDA(cudaStreamSynchronize(st));
     float ms = 0;
     cudaEventElapsedTime(&ms, e0, e1);
@@ -2147,7 +2149,7 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
         stats->rays_tail = hs[kRaysT];
     }
     for (cudaEvent_t e : ev) cudaEventDestroy(e);
-    if (cfg->use_cache) KGK_TRY(nrc_finish(*s->nrc, st, nullptr));
+    if (cfg->use_cache) KGK_TRY(nrc_status(*s->nrc, cache_status, st));
     if (hs[kOverflow])
         return fail(KGK_ERR_DEVICE_CHECK, "kgk_render: " + std::to_string(hs[kOverflow]) +
                                               " traversals overflowed their stack");
