@@ -1312,13 +1312,13 @@ kgk_status kgk_nrc_set_weights(kgk_scene *s, const float *w, size_t n) {
     NrcState &N = *s->nrc;
     if (!w || n != (size_t)N.params)
         return fail(KGK_ERR_INVALID_ARGUMENT, "kgk_nrc_set_weights: expected " + std::to_string(N.params) + " floats");
-    // On the legacy stream, after what made the weights there; the host may be back
-    // before the copy is done, and the scene's stream does not wait for that one.
+    // All on the legacy stream, after what made the weights there: the host may be
+    // back before the copy is done, and the scene's stream does not wait for that one.
+    KGK_CUDA(cudaStreamSynchronize(s->stream));  // nothing reads the old ones any more
     KGK_CUDA(cudaMemcpy(N.w, w, n * sizeof(float), is_device_ptr(w) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
-    KGK_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
-    make_image(N, s->stream);
+    make_image(N, cudaStreamLegacy);
     KGK_CUDA(cudaGetLastError());
-    KGK_CUDA(cudaStreamSynchronize(s->stream));
+    KGK_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     return KGK_OK;
 }
 
