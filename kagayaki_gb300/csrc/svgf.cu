@@ -76,9 +76,10 @@ constexpr float kLog2e = 1.44269504088896341f;
 // least (x = -100: 2^-15 of 2^-100), and never more than 2^-21 in absolute terms,
 // as 2^x |x| ln 2 is at most 1 / e.
 // The quotient is formed with both sides a quarter: __fdividef gives 0 for a
-// divisor above 2^126, which slopes of 10^38 reach.
-__device__ __forceinline__ float depth_arg(float d, float nd, float slope) {
-    return __fdividef(-0.25f * kLog2e * fabsf(d - nd), fmaf(0.25f, fabsf(slope), 0.25f * kS));
+// divisor above 2^126, which slopes of 10^38 reach.  slope4: a quarter of the
+// slope, from gradients scaled once per pixel.
+__device__ __forceinline__ float depth_arg(float d, float nd, float slope4) {
+    return __fdividef(-0.25f * kLog2e * fabsf(d - nd), fabsf(slope4) + 0.25f * kS);
 }
 __device__ __forceinline__ float normal_w(float3 n, float3 m) {
     float c = fmaxf(0.0f, dot3(n, m));
@@ -288,7 +289,7 @@ __global__ void __launch_bounds__(256) k_c_var(CompatArgs a) {
     if (sp && !reset) {
         const float4 cn = s_nd[c];
         const float3 n = f3(cn);
-        const float gzx = a.gz[2 * p], gzy = a.gz[2 * p + 1];
+        const float gzx = 0.25f * a.gz[2 * p], gzy = 0.25f * a.gz[2 * p + 1];
         float s1 = 0, s2 = 0, sw = 0;
         for (int kx = -3; kx <= 3; ++kx) {
             const int nx = x + kx;
@@ -424,7 +425,7 @@ struct CompatPx {
     float4 af, dcl;   // albedo and filter flag, own demodulated radiance
     int2 om;          // own material and variance
     float3 n;
-    float d, l, gx, gy;
+    float d, l, gx, gy;  // gx, gy: a quarter of the depth gradient
     float rl;         // the luminance weight's factor of |l - nl|
     float bright;     // a tap brighter than this is left out
     float3 srad;
@@ -440,8 +441,8 @@ struct CompatPx {
         d = nd.w;
         l = dm.w;
         const float2 g = reinterpret_cast<const float2 *>(a.gz)[p];
-        gx = g.x;
-        gy = g.y;
+        gx = 0.25f * g.x;
+        gy = 0.25f * g.y;
         rl = __fdividef(-kLog2e, 4.0f * a.sd[p] + kS);
         // SVGF.cuh:405-411, whose first two bounds compare in double
         bright = (double)l > 0.5 ? 5 * l : (double)l > 0.1 ? 50 * l : l > kS ? 100 * l : INFINITY;
