@@ -224,8 +224,9 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 // and w + 4 share one).  Width 128: 824 -> 1160 TFLOP/s (a 4K frame's queries
 // 240 -> 169 us; one warpgroup a tile 183).  Width 64, 2^21 queries: 107 ->
 // 102 us (five tiles without the overlapped encoding 110, two warpgroups a tile
-// 106); leaving out the encoding, three of four MMAs or the query loads there
-// takes 8 % each: no one of them bounds it, four tiles' latency does.
+// 106); there leaving out the encoding takes 8 %, three of four MMAs 10 %, the
+// query loads 6 %: no one of them bounds it, four tiles' latency does (tensor pipe
+// 38 % active, 56 % at width 128).
 namespace tc {
 template <int W>
 struct Ti {

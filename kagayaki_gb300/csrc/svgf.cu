@@ -402,14 +402,14 @@ __global__ void k_c_gauss(CompatArgs a) {
 // luminance (dm, written by the pass before) instead of being divided by its
 // albedo at every tap.  The filtered image and the records' flags and history
 // take their last pass's values, so they are stored once, in k_c_final.
-// Instruction issue bounds a pass (two IEEE divisions and two expf a tap
-// before, one reciprocal and one ex2 now), then shared memory (40 B a tap).
-// 1080p: a pass 202 / 195 / 201 / 247 / 244 us at steps 1 / 2 / 4 / 8 / 16 ->
-// 98 / 99 / 118 / 144 / 146, with two pixels a thread at the last two 123 /
-// 123; the passes over the 112-byte records before and after 1.19 -> 0.45 ms;
-// the call 6.47 -> 3.67 ms.  Error
-// against 64 bits over 64 x 64 to 2560 x 1440, with and without motion:
-// 3.6e-7 to 5.4e-7 before and after.
+// Instruction issue (two IEEE divisions and two expf a tap before, one
+// reciprocal and one ex2 now) and shared memory (40 B a tap) bound a pass on
+// tiles, at 66 % and 89 % of their peaks.  1080p: a pass 202 / 195 / 201 / 247 /
+// 244 us at steps 1 / 2 / 4 / 8 / 16 -> 96 / 97 / 115 / 144 / 146, with two pixels
+// a thread at the last two 118 / 117; the passes over the 112-byte records before
+// and after 1.19 -> 0.45 ms; the call 6.35 -> 3.57 ms.  Error against 64 bits, 300
+// x 200 to 1920 x 1080, with and without motion: 2e-7 to 2e-6 on both sides, the
+// same on the same inputs (and 3e-4 where a brightness test falls the other way).
 struct CompatIO {
     const kgk_vec *Rin;
     kgk_vec *Rout;
@@ -564,8 +564,9 @@ __global__ void k_c_atrous(CompatArgs a, CompatIO io, int stage) {
 // its pixels and a halo of 2 * step in shared memory - guide, demodulated
 // radiance, material and variance - then filters from there.  Entries outside
 // the image are never read (the tap's bounds test comes first).  Two pixels a
-// thread, as in the rows below, measured slower here (98 / 99 / 118 us a pass
-// to 110 / 113 / 122: half the blocks, 76 registers, for little less staging).
+// thread, as in the rows below, measured slower here (98 / 99 / 118 us a pass at
+// the time to 110 / 113 / 122: half the blocks, 76 registers, for little less
+// staging).
 template <int kStep> struct CTile {
     static constexpr int R = 2 * kStep, SX = kCTX + 2 * R, SY = kCTY + 2 * R, N = SX * SY;
     static constexpr size_t kSmem = (size_t)N * (2 * sizeof(float4) + sizeof(int2));

@@ -345,8 +345,8 @@ __device__ __forceinline__ bool trace_any(const WideNode *__restrict__ nodes, un
 // warp tests 32 pairs at a time, whichever rays they belong to, from a shared
 // copy of the rays; a ray's closest hit is kept in shared memory too, so the
 // lane's registers hold only what node visits need.
-// Instruction issue bounds it (76 % of slots on incoherent rays, DRAM below
-// 10 %).  On the 5.2M-triangle frame a step's own-triangle loop ran 2.6 times
+// Instruction issue bounds it (68 to 72 % of slots on incoherent rays, the ALU
+// pipe at 53 %, DRAM below 10 %).  On the 5.2M-triangle frame a step's own-triangle loop ran 2.6 times
 // at 6.9 lanes; pairs run 1.3 times at 14.2.  With the leaf field and the
 // paired multiply-adds of node_intersect, closest-hit batches (2^22 rays, 1.3M
 // triangles) 524 -> 479 us, the 64-sample 1080p frame 93.3 -> 89.6 ms, two
