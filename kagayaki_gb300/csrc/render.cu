@@ -1321,9 +1321,8 @@ __device__ __forceinline__ void compat_flush(const Params &P, const CompatCount 
 
 // A pixel per thread (slots in 8 x 4 tiles), the block going through the
 // launch's samples one after another; `first`: of the call, else the frame's sums
-// go on.  The seed chain orders a pixel's own
-// samples only (render.cuh:19,29,42), so no block waits for another's longest
-// path and a sample needs no launches.  Cornell box, 256 x 256, 16 samples:
+// go on.  The seed chain orders a pixel's own samples only (render.cuh:19,29,42),
+// so no block waits for another's longest path and a sample needs no launches.  Cornell box, 256 x 256, 16 samples:
 // 3.36 -> 2.44 ms (a wave of three launches per sample before; the same with
 // a barrier per phase 2.81; a warp going through its 32 pixels' samples alone
 // 3.30).
@@ -1900,10 +1899,10 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
         P.spp_wave = 1;
         // one block per SM, whose warps are then all in step
         const int per = std::min(kCompatThreads, std::max(32, ((npx + R.sms - 1) / R.sms + 31) & ~31));
-        for (int done = 0; done < cfg->spp; done += kCompatSamples) {
+        for (int left = cfg->spp; left > 0; left -= kCompatSamples) {
             KGK_TRY(stage_begin(3));
-            k_compat<<<(npx + per - 1) / per, per, 0, st>>>(P, std::min(kCompatSamples, cfg->spp - done), max_bounces,
-                                                            R.frame, R.acc_sum, R.acc_sq, cfg->accumulate, done == 0);
+            k_compat<<<(npx + per - 1) / per, per, 0, st>>>(P, std::min(kCompatSamples, left), max_bounces, R.frame,
+                                                            R.acc_sum, R.acc_sq, cfg->accumulate, left == cfg->spp);
             KGK_TRY(stage_end());
             KGK_CUDA(cudaGetLastError());
             ++launches;
