@@ -518,4 +518,87 @@ __device__ __forceinline__ bool warp_step(const WideNode *__restrict__ nodes, un
     return false;
 }
 
+// The same step with each lane testing the triangles of its own visit, an occluded
+// ray none after its first hit.  In closed rooms nearly every ray has its hit in
+// the first node it meets, and listing all of that node's triangles in shared
+// memory is what the pairs cost there.  Same nodes, culling and hit rules.
+struct OwnRay {
+    RayPre r;
+    uint2 group;
+    int sp;
+    float best_t;
+    int best_id;  // kNoHit: none yet
+};
+constexpr int kNoHit = 0x7fffffff;
+
+__device__ __forceinline__ void own_init(OwnRay &c, float3 o, float3 d, float tmax) {
+    c.r = make_ray(o, d);
+    c.group = make_uint2(0u, 0x80000000u);
+    c.sp = 0;
+    c.best_t = tmax;
+    c.best_id = kNoHit;
+}
+
+// Returns true when the lane's ray is finished.
+template <bool kAny, bool kCount>
+__device__ __forceinline__ bool own_step(const WideNode *__restrict__ nodes, unsigned n_nodes,
+                                         const float4 *__restrict__ tri, unsigned n_tris, OwnRay &c, TravStack &stk,
+                                         TravStats &st) {
+    uint2 tg = make_uint2(0u, 0u);
+    unsigned leaves = 0u;
+#pragma unroll 1
+    for (int visit = 0; visit < kNodesPerStep && tg.y == 0u; ++visit) {
+        if ((c.group.y & 0xff000000u) == 0u) {
+            if (c.sp == 0) break;
+            c.group = stk.e[--c.sp];
+        }
+        const unsigned hits_imask = c.group.y;
+        const int child_bit = 31 - __clz(hits_imask & 0xff000000u);
+        const unsigned base = c.group.x;
+        c.group.y &= ~(1u << child_bit);
+        if (c.group.y & 0xff000000u) {
+            if (c.sp < kTravStack) stk.e[c.sp++] = c.group;
+            else st.overflow = 1;
+        }
+        const unsigned slot = (unsigned)(child_bit - 24) ^ octant_xor(c.r.oct);
+        const unsigned rel = __popc(hits_imask & ~(0xffffffffu << slot));
+        if (base + rel >= n_nodes) { st.overflow = 2; return true; }
+        const WideNode *nd = nodes + base + rel;
+        const float4 n0 = __ldg(&nd->n0), n1 = __ldg(&nd->n1), n2 = __ldg(&nd->n2), n3 = __ldg(&nd->n3),
+                     n4 = __ldg(&nd->n4);
+        if (kCount) ++st.nodes;
+        const unsigned hm = node_intersect(c.r.o, c.r.inv, c.r.oct, c.best_t, n0, n1, n2, n3, n4);
+        leaves = __float_as_uint(n1.z);
+        c.group = make_uint2(__float_as_uint(n1.x), (hm & 0xff000000u) | leaves >> 24);
+        tg = make_uint2(__float_as_uint(n1.y), hm & 0x00ffffffu);
+    }
+    while (tg.y != 0u) {
+        const int k = __ffs(tg.y) - 1;
+        tg.y &= tg.y - 1u;
+        const int ti = (int)tg.x + __popc(leaves & ((1u << k) - 1u));
+        if ((unsigned)ti >= n_tris) { st.overflow = 2; return true; }
+        const float4 a = __ldg(&tri[3 * ti]), b = __ldg(&tri[3 * ti + 1]), cc = __ldg(&tri[3 * ti + 2]);
+        if (kCount) ++st.tris;
+        float t, u, v;
+        if (!tri_intersect(c.r, a, b, cc, &t, &u, &v)) continue;
+        ref_distance(c.r, a, b, cc, &t, &u, &v);
+        if (!(t >= kTMin)) continue;
+        const int id = __float_as_int(a.w);
+        if (kAny) {
+            if (t < c.best_t) {
+                c.best_id = id;
+                return true;
+            }
+        } else if (t < c.best_t || (t == c.best_t && id < c.best_id)) {
+            c.best_t = t;
+            c.best_id = id;
+        }
+    }
+    if ((c.group.y & 0xff000000u) == 0u) {
+        if (c.sp == 0) return true;
+        c.group = stk.e[--c.sp];
+    }
+    return false;
+}
+
 }  // namespace kgk
