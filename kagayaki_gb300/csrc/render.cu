@@ -124,8 +124,9 @@ constexpr int kTailRefill = 8;
 constexpr int kCompatTris = 1024, kCompatThreads = 512, kCompatSamples = 64;
 // ... and the largest scene of which it renders one or two samples of a small image.
 constexpr int kCompatFewTris = 128;
-// The largest scene whose waves trace by k_extend_loop and k_shadow_loop.
-constexpr int kLoopTris = 1024;
+// The largest scenes whose waves trace by k_extend_loop and k_shadow_loop: their
+// first bounce, and all bounces.
+constexpr int kLoopTris = 1024, kLoopAllTris = 256;
 // Deferred shadow rays of the tail (unbiased estimator without the cache):
 // the first kDeferBounces bounces of a tail path leave their face-light and
 // environment shadow rays in fixed slots (path, bounce, kind) instead of
@@ -1919,7 +1920,18 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
     //   2,562  1.44 : 1.39, 1.06 : 1.02, 0.80 : 0.76, 5.01 : 4.98 (spheres under a sky)
     //          1.58 : 1.54, 1.08 : 1.05, 0.73 : 0.73, 3.60 : 3.95 (two spheres)
     //          1.65 : 1.59, 1.15 : 1.12, 0.98 : 0.94, 4.66 : 4.69 (eight spheres)
-    // Even between 962 and 1,282 triangles, but for large unbiased waves.
+    // Even between 962 and 1,282 triangles of spheres, but for large unbiased waves.
+    // What the loops gain there is the first bounce's, whose rays are alike; later
+    // ones wait for a warp's longest ray.  All bounces : the first, then pairs :
+    // pairs, the reference's estimator at 640 x 480 x 4, the unbiased one at 1080p x
+    // 8, closed rooms of
+    //   84     2.54 : 2.82 : 2.90, 21.1 : 23.7 : 24.3
+    //   144    2.62 : 2.82 : 2.87, 21.6 : 22.8 : 23.2
+    //   264    3.17 : 3.27 : 3.34, 27.4 : 26.7 : 27.1
+    //   504    3.83 : 3.70 : 3.75, 33.4 : 29.9 : 30.2
+    //   1,020  4.16 : 4.09 : 4.14, 35.7 : 32.0 : 32.3
+    // and of spheres, 322 1.25 : 1.25 : 1.28, 3.40 : 3.42 : 3.81, 642 1.38 : 1.33 : 1.37,
+    // 3.54 : 3.48 : 3.86.
     // Blocks of large waves finish at different times; three times what fits at
     // once evens them out, but costs small ones.  Paths of a wave, one : three
     // times, on the box: 0.31M 0.514 : 0.544 (unbiased), 1.54 : 1.59 (the
@@ -1927,11 +1939,11 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
     // 0.793 : 0.790, 1.33 : 1.34; 1.23M 1.110 : 1.108; 1.31M 2.23 : 2.19 (the
     // reference's); 1.84M 1.236 : 1.214; 2.07M 1.351 : 1.316, 2.52 : 2.48; 16.6M
     // 8.01 : 7.77.
-    const bool loops = s->dev.n_tris <= kLoopTris;
+    const auto loops = [&](int bounce) { return s->dev.n_tris <= (bounce == 0 ? kLoopTris : kLoopAllTris); };
     const int loop_grid = (size_t)npx * std::min(spw, (int)cfg->spp) >= (1u << 20) ? 3 * grid : grid;
-    auto shadow = [&](int q) {
+    auto shadow = [&](int q, bool loop) {
         const int ci = q ? kSH1 : kSH0, fi = q ? kFS1 : kFS0;
-        if (loops) k_shadow_loop<<<loop_grid, 128, 0, sh_st>>>(P, ci, R.sh_o[q], R.sh_d[q], R.sh_c[q]);
+        if (loop) k_shadow_loop<<<loop_grid, 128, 0, sh_st>>>(P, ci, R.sh_o[q], R.sh_d[q], R.sh_c[q]);
         else k_shadow<<<grid, 128, 0, sh_st>>>(P, ci, fi, R.sh_o[q], R.sh_d[q], R.sh_c[q]);
     };
     for (int done = by_pixel ? cfg->spp : 0, wave = 0; done < cfg->spp; done += spw, ++wave) {
@@ -1986,10 +1998,10 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
             KGK_CUDA(cudaMemsetAsync(R.cnt + kMQ, 0, (kDQ + 1 - kMQ) * sizeof(int), st));
             KGK_CUDA(cudaMemsetAsync(R.cnt + nidx, 0, sizeof(int), st));
             KGK_TRY(stage_begin(0));
-            if (cfg->count_work)
-                (loops ? k_extend_loop<true> : k_extend<true>)<<<loops ? loop_grid : grid, 128, 0, st>>>(P, cidx, n, R.mq, R.lq, R.dq);
-            else
-                (loops ? k_extend_loop<false> : k_extend<false>)<<<loops ? loop_grid : grid, 128, 0, st>>>(P, cidx, n, R.mq, R.lq, R.dq);
+            const bool loop = loops(b);
+            auto *extend = cfg->count_work ? (loop ? k_extend_loop<true> : k_extend<true>)
+                                           : (loop ? k_extend_loop<false> : k_extend<false>);
+            extend<<<loop ? loop_grid : grid, 128, 0, st>>>(P, cidx, n, R.mq, R.lq, R.dq);
             KGK_TRY(stage_end());
             ++extend_launches;
             // shading adds to the radiance the previous shadow passes wrote and
@@ -2030,10 +2042,10 @@ kgk_status kgk_render(kgk_scene *s, const kgk_camera *cam, const kgk_camera *pre
             KGK_CUDA(cudaStreamWaitEvent(sh_st, R.shaded, 0));
             KGK_TRY(stage_begin(2, sh_st));
             if (face_lights) {
-                shadow(0);
+                shadow(0, loop);
                 ++launches;
             }
-            shadow(1);
+            shadow(1, loop);
             KGK_TRY(stage_end(sh_st));
             KGK_CUDA(cudaEventRecord(R.shadowed, sh_st));
             shadow_pending = true;

@@ -55,3 +55,22 @@ def test_both_sides_of_the_lines(n_tris, W, H, spp):
     """Triangles and samples, paths of a wave of the tail kernel (363 x 361 is the
     last size), pixels: as with more triangles than the kernel takes."""
     same(rendered(n_tris - 36, W, H, spp), rendered(2000, W, H, spp))
+
+
+@pytest.mark.parametrize("kind", ["cornell", "disney"])
+@pytest.mark.parametrize("n_tris", [256, 257, 1024, 1025])
+def test_lines_of_the_loops(kind, n_tris):
+    """Waves of 262,144 paths, whose bounces trace by loops, by loops and then by the
+    warp's pairs, or by pairs: unbiased frames as with many more triangles."""
+    from kagayaki_gb300 import ESTIMATOR_UNBIASED
+    from test_compat_routes_gpu import far_away
+    tris, mats, c, tex, env = scenes.parity_scene(kind)
+    got = []
+    for n in (n_tris, 4000):
+        with Scene(far_away(tris, n - len(tris)), mats, textures=tex, env=env) as s:
+            s.build_bvh()
+            cam = camera_setup(c["origin"], c["dist"], c["rot"], 256)
+            img, st = s.render(cam, 512, 256, spp=2, estimator=ESTIMATOR_UNBIASED, accumulate=False)
+            got.append((img.copy(), st["extend_launches"], st["rays_closest"], st["rays_shadow"]))
+    assert got[0][1] >= 2 and got[0][1:] == got[1][1:]
+    assert np.array_equal(got[0][0], got[1][0], equal_nan=True)
